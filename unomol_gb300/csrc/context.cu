@@ -22,6 +22,7 @@
 
 #include "../../include/unomol_gb300.h"
 #include "ctx_view.h"
+#include "fock_df64.cuh"
 #include "fock_dispatch.cuh"
 #include "fock_kernels.cuh"
 #include "setup.h"
@@ -81,14 +82,23 @@ struct UnomolCtx {
     int* d_launch_bp = nullptr;  // per class launch: first block pair, block pairs
     float* d_dmax = nullptr;
     double skip_cut = 1e-13;
+    // the FP64 build's own split of every staircase row at SPLIT_CUT (set by the geometry alone): quartets
+    // above it (FP64 kernels) and below it (pairs of floats), with their totals per class launch
+    long long *d_pre_hi = nullptr, *d_pre_lo = nullptr, *d_cnt_hi = nullptr, *d_cnt_lo = nullptr;
+    long long *d_begin_hi = nullptr, *d_begin_lo = nullptr, *d_total_hi = nullptr, *d_total_lo = nullptr;
+    int* d_mseg_hi = nullptr;
+    float* d_one = nullptr;  // 1.0: the split's density bound
+    std::vector<long long> total_hi, total_lo;
     // device buffers
     ShellPair* d_pairs = nullptr;
     PrimPair* d_prims = nullptr;
     PrimPair32* d_prims32 = nullptr;
+    PrimPairDF* d_primsdf = nullptr;
     BlockPair* d_bps = nullptr;
     long long* d_prefix = nullptr;
     double* d_rys = nullptr;
     float* d_rys32 = nullptr;
+    float* d_rysdf = nullptr;
     double *d_Pa = nullptr, *d_Pb = nullptr, *d_Ta = nullptr, *d_Tb = nullptr;
     double *d_Ga = nullptr, *d_Gb = nullptr, *d_pk_a = nullptr, *d_pk_b = nullptr;
     float* d_pmax = nullptr;
@@ -299,6 +309,16 @@ int build_worklists(UnomolCtx* ctx) {
             ctx->d_total64 = c.take<long long>(NPAIRCLASS * NPAIRCLASS);
             ctx->d_total32 = c.take<long long>(NPAIRCLASS * NPAIRCLASS);
             ctx->d_launch_bp = c.take<int>(2 * NPAIRCLASS * NPAIRCLASS);
+            ctx->d_pre_hi = c.take<long long>(nrows);
+            ctx->d_pre_lo = c.take<long long>(nrows);
+            ctx->d_mseg_hi = c.take<int>(nrows);
+            ctx->d_cnt_hi = c.take<long long>(nall);
+            ctx->d_cnt_lo = c.take<long long>(nall);
+            ctx->d_begin_hi = c.take<long long>(nall);
+            ctx->d_begin_lo = c.take<long long>(nall);
+            ctx->d_total_hi = c.take<long long>(2 * NPAIRCLASS * NPAIRCLASS);  // above SPLIT_CUT, then below
+            ctx->d_total_lo = ctx->d_total_hi ? ctx->d_total_hi + NPAIRCLASS * NPAIRCLASS : nullptr;
+            ctx->d_one = c.take<float>(1);
         };
         Carve lay;
         lists(lay);
@@ -378,6 +398,22 @@ int build_worklists(UnomolCtx* ctx) {
         CU(cudaMemsetAsync(ctx->d_c64, 0, sizeof(long long) * nr, s));
         CU(cudaMemsetAsync(ctx->d_c32, 0, sizeof(long long) * nr, s));
         CU(cudaMemsetAsync(ctx->d_mseg, 0, sizeof(int) * nr, s));
+        // the FP64 build's split at SPLIT_CUT: the same passes as a screened build's, with a density bound of
+        // one and nothing skipped, once per set-up; the totals size the launches
+        const float one = 1.f;
+        const int nl = (int)ctx->launches.size();
+        long long tot2[2 * NPAIRCLASS * NPAIRCLASS];
+        CU(cudaMemcpyAsync(ctx->d_one, &one, sizeof(float), cudaMemcpyHostToDevice, s));
+        CU(wl_split_rows(ctx->d_pairs, ctx->d_bps, ctx->d_rowbp, ctx->d_prefix, nrows, ctx->d_one, SPLIT_CUT, 0.0, ctx->d_c64,
+                         ctx->d_c32, ctx->d_mseg_hi, s));
+        CU(wl_scan_rows(ctx->d_bps, (int)nbp, ctx->d_c64, ctx->d_c32, ctx->d_pre_hi, ctx->d_pre_lo, ctx->d_cnt_hi,
+                        ctx->d_cnt_lo, s));
+        CU(wl_scan_launches(ctx->d_launch_bp, nl, ctx->d_cnt_hi, ctx->d_cnt_lo, ctx->d_begin_hi, ctx->d_begin_lo,
+                            ctx->d_total_hi, ctx->d_total_lo, s));
+        CU(cudaMemcpyAsync(tot2, ctx->d_total_hi, sizeof(tot2), cudaMemcpyDeviceToHost, s));
+        CU(cudaStreamSynchronize(s));
+        ctx->total_hi.assign(tot2, tot2 + nl);
+        ctx->total_lo.assign(tot2 + NPAIRCLASS * NPAIRCLASS, tot2 + NPAIRCLASS * NPAIRCLASS + nl);
     }
     CU(cudaStreamSynchronize(s));
     return UNOMOL_OK;
@@ -405,6 +441,7 @@ int build_setup(UnomolCtx* ctx) {
             ctx->d_pairs = c.take<ShellPair>(P);
             ctx->d_prims = c.take<PrimPair>(nprims);
             ctx->d_prims32 = c.take<PrimPair32>(nprims);
+            ctx->d_primsdf = c.take<PrimPairDF>(nprims);
         };
         Carve lay;
         recs(lay);
@@ -543,8 +580,17 @@ int build_setup(UnomolCtx* ctx) {
         CU(cudaMemcpyAsync(a.bbegin, ctx->block_begin.data(), sizeof(int) * nb, cudaMemcpyHostToDevice, s));
         CU(cudaMemcpyAsync(a.bcount, ctx->block_count.data(), sizeof(int) * nb, cudaMemcpyHostToDevice, s));
         CU(cudaMemcpyAsync(a.bprim, bprim.data(), sizeof(long long) * nb, cudaMemcpyHostToDevice, s));
+        double origin[3];  // the middle of the molecule's box
+        for (int k = 0; k < 3; ++k) {
+            double lo = ctx->centers[k], hi = lo;
+            for (int c = 1; c < ctx->ncen; ++c) {
+                lo = std::min(lo, ctx->centers[3 * c + k]);
+                hi = std::max(hi, ctx->centers[3 * c + k]);
+            }
+            origin[k] = 0.5 * (lo + hi);
+        }
         CU(setup_interleave_prims(ctx->d_pairs, P, a.bbegin, a.bcount, a.bprim, nb, a.prims_c, a.prims32_c, ctx->d_prims,
-                                  ctx->d_prims32, s));
+                                  ctx->d_prims32, ctx->d_primsdf, origin, s));
         CU(cudaStreamSynchronize(s));  // the host arrays above are copied from pageable memory
     }
     return build_worklists(ctx);
@@ -607,6 +653,53 @@ static cudaError_t launch_class_kernel(const UnomolCtx* ctx, const ClassLaunch& 
     return launch_fock_generic(la, lb, lc, ld, uhf, fp32, A, ctx->nt, ctx->d_rys, ctx->d_rys32, s);
 }
 
+// One class of an FP64 build: launches of few quartets in FP64 with a warp per quartet; otherwise the
+// quartets at or above SPLIT_CUT in FP64 on stream sh (a few lanes per quartet) and those below it in pairs
+// of floats on stream sl.  Classes without those kernels (MD, f and g shells, large d classes) as one launch.
+cudaError_t launch_plain_class(const UnomolCtx* ctx, size_t li, bool uhf, FockArgs A, cudaStream_t sh, cudaStream_t sl,
+                               int& launches) {
+    const ClassLaunch& L = ctx->launches[li];
+    A.bps = ctx->d_bps + L.bp_begin;
+    A.prefix = ctx->d_prefix;
+    A.nbp = L.nbp;
+    A.nwork = L.nwork;
+    A.mode = 0;
+    const int lsum = pc_la(L.bc) + pc_lb(L.bc) + pc_la(L.kc) + pc_lb(L.kc);
+    if (ctx->eri_method == UNOMOL_ERI_MD || lsum > 8 || !fock_mixed_fused(L.bc, L.kc)) {
+        ++launches;
+        return launch_class_kernel(ctx, L, uhf, false, A, sl);
+    }
+    // a warp per quartet up to 32 quartets per SM (one wave of 8 CTAs of 4 warps); above, one lane per quartet
+    // starts to fill the SMs
+    const long long few = (long long)ctx->nsm * 32;
+    if (L.nwork <= few) {
+        ++launches;
+        return launch_fock_fp64_group(L.bc, L.kc, uhf, A, L.nwork, false, 32, ctx->nt, ctx->d_rys, sl);
+    }
+    A.dyn_mseg = ctx->d_mseg_hi;
+    const long long hi = ctx->total_hi[li], lo = ctx->total_lo[li];
+    cudaError_t e = cudaSuccess;
+    if (hi > 0) {
+        A.mode = 3;
+        A.dyn_prefix = ctx->d_pre_hi;
+        A.dyn_count = ctx->d_cnt_hi + L.bp_begin;
+        A.dyn_begin = ctx->d_begin_hi + L.bp_begin;
+        A.dyn_total = ctx->d_total_hi + li;
+        e = launch_fock_fp64_group(L.bc, L.kc, uhf, A, hi, true, hi <= few ? 32 : 4, ctx->nt, ctx->d_rys, sh);
+        ++launches;
+    }
+    if (e == cudaSuccess && lo > 0) {
+        A.mode = 4;
+        A.dyn_prefix = ctx->d_pre_lo;
+        A.dyn_count = ctx->d_cnt_lo + L.bp_begin;
+        A.dyn_begin = ctx->d_begin_lo + L.bp_begin;
+        A.dyn_total = ctx->d_total_lo + li;
+        e = launch_fock_df64(L.bc, L.kc, uhf, A, lo, ctx->nt, ctx->d_rysdf, sl);
+        ++launches;
+    }
+    return e;
+}
+
 // Fock build from the stored integral matrix (unomol_gpu_store_integrals / _store_records).
 int store_build(UnomolCtx* ctx, const double* dPa, const double* dPb, double* dGa, double* dGb, cudaStream_t s) {
     if (dPb && store_kind(ctx->store) != UNOMOL_STORE_UHF)
@@ -645,6 +738,7 @@ int fock_device(UnomolCtx* ctx, const double* dPa, const double* dPb, double* dG
     A.pairs = ctx->d_pairs;
     A.prims = ctx->d_prims;
     A.prims32 = ctx->d_prims32;
+    A.primsdf = ctx->d_primsdf;
     A.nbf = n;
     A.Pa = ctx->d_Pa;
     A.Pb = uhf ? ctx->d_Pb : nullptr;
@@ -713,12 +807,12 @@ int fock_device(UnomolCtx* ctx, const double* dPa, const double* dPb, double* dG
     cudaStream_t ls[2] = {s, s};  // streams of the FP64 and FP32 launches (plain builds: alternate classes)
     if (!ctx->counting) {
         CU(cudaEventRecord(ctx->fork, s));
-        ls[0] = ctx->part_stream[mixed ? 0 : 1];
-        ls[1] = ctx->part_stream[mixed ? 1 : 2];
+        ls[0] = ctx->part_stream[0];
+        ls[1] = ctx->part_stream[1];
         for (int k = 0; k < 2; ++k) CU(cudaStreamWaitEvent(ls[k], ctx->fork, 0));
     }
-    auto launch_class = [&](const ClassLaunch& L, bool fp32, bool side = false) -> cudaError_t {
-        return launch_class_kernel(ctx, L, uhf, fp32, A, ls[(fp32 || side) ? 1 : 0]);
+    auto launch_class = [&](const ClassLaunch& L, bool fp32) -> cudaError_t {
+        return launch_class_kernel(ctx, L, uhf, fp32, A, ls[fp32 ? 1 : 0]);
     };
     for (size_t lk = 0; lk < ctx->launches.size(); ++lk) {
         const size_t li = ctx->reverse_launches ? ctx->launches.size() - 1 - lk : lk;
@@ -729,9 +823,7 @@ int fock_device(UnomolCtx* ctx, const double* dPa, const double* dPb, double* dG
         A.nwork = L.nwork;
         A.counter_base = (L.bc * NPAIRCLASS + L.kc) * 32;  // FP32 launches use the second half
         if (!mixed) {
-            A.mode = 0;
-            CU(launch_class(L, false, (li & 1) != 0));
-            ++launches;
+            CU(launch_plain_class(ctx, li, uhf, A, ls[0], ls[(lk & 1) ? 1 : 0], launches));
         } else {
             A.mode = 1;
             A.dyn_prefix = ctx->d_pre64;
@@ -916,12 +1008,14 @@ constexpr int RYS64_LEN = rys_table_len(RysStride<double>::value, RYS_H);
 constexpr int RYS32_LEN = rys_table_len(RysStride<float>::value, RYS32_H);
 static __device__ __align__(32) double g_rys64[RYS64_LEN];  // 64-byte rows: two 256-bit loads each
 static __device__ __align__(32) float g_rys32[RYS32_LEN];  // 32-byte rows: one 256-bit load each
+static __device__ __align__(64) float g_rysdf[DF_TABLE_LEN];  // 64-byte rows: two 256-bit loads each
 constexpr int RYS_MAX_DEVICES = 64;
 double* g_rys64_ptr[RYS_MAX_DEVICES] = {nullptr};
 float* g_rys32_ptr[RYS_MAX_DEVICES] = {nullptr};
+float* g_rysdf_ptr[RYS_MAX_DEVICES] = {nullptr};
 std::mutex g_rys_mu;
 
-int rys_tables(int dev, double*& d64, float*& d32, std::string& err) {
+int rys_tables(int dev, double*& d64, float*& d32, float*& ddf, std::string& err) {
     static_assert(rys_table_len(RYS_DEG + 1, RYS_H) == RYS_TABLE_SIZE + 50, "layout of rys_tables.inc");
     static_assert(rys_table_len(RYS32_DEG + 1, RYS32_H) == RYS32_TABLE_SIZE + 50, "layout of rys_tables.inc");
     if (dev < 0 || dev >= RYS_MAX_DEVICES) {
@@ -946,10 +1040,13 @@ int rys_tables(int dev, double*& d64, float*& d32, std::string& err) {
                 t32[h32 + n * 5 + i] = (float)RYS_HERMITE_X_H[n][i];
                 t32[h32 + 25 + n * 5 + i] = (float)RYS_HERMITE_W_H[n][i];
             }
-        void *p64 = nullptr, *p32 = nullptr;
+        const std::vector<float> tdf = df_rys_tables();
+        void *p64 = nullptr, *p32 = nullptr, *pdf = nullptr;
         cudaError_t e = cudaMemcpyToSymbol(g_rys64, t64.data(), sizeof(double) * t64.size());
         if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_rys32, t32.data(), sizeof(float) * t32.size());
+        if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_rysdf, tdf.data(), sizeof(float) * tdf.size());
         if (e == cudaSuccess) e = cudaGetSymbolAddress(&p64, g_rys64);
+        if (e == cudaSuccess) e = cudaGetSymbolAddress(&pdf, g_rysdf);
         if (e == cudaSuccess) e = cudaGetSymbolAddress(&p32, g_rys32);
         if (e != cudaSuccess) {
             err = std::string("Rys tables: ") + cudaGetErrorString(e);
@@ -957,9 +1054,11 @@ int rys_tables(int dev, double*& d64, float*& d32, std::string& err) {
         }
         g_rys64_ptr[dev] = static_cast<double*>(p64);
         g_rys32_ptr[dev] = static_cast<float*>(p32);
+        g_rysdf_ptr[dev] = static_cast<float*>(pdf);
     }
     d64 = g_rys64_ptr[dev];
     d32 = g_rys32_ptr[dev];
+    ddf = g_rysdf_ptr[dev];
     return UNOMOL_OK;
 }
 
@@ -982,7 +1081,7 @@ int init_device(UnomolCtx* ctx, int np) {
     CU(cudaEventCreateWithFlags(&ctx->fork, cudaEventDisableTiming));
     for (auto& e : ctx->join) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     {
-        const int rc = rys_tables(ctx->dev, ctx->d_rys, ctx->d_rys32, ctx->err);
+        const int rc = rys_tables(ctx->dev, ctx->d_rys, ctx->d_rys32, ctx->d_rysdf, ctx->err);
         if (rc) return fail(ctx, rc, ctx->err);
     }
     // the basis in one allocation (status flag, shell arrays, exponents, coefficients, centres), from a
@@ -1373,6 +1472,7 @@ extern "C" int unomol_gpu_fock_rhf_noalloc(UnomolCtx* ctx, const double* dP, dou
     A.pairs = ctx->d_pairs;
     A.prims = ctx->d_prims;
     A.prims32 = ctx->d_prims32;
+    A.primsdf = ctx->d_primsdf;
     A.nbf = n;
     A.Pa = Pfull;
     A.Pb = nullptr;
@@ -1385,16 +1485,8 @@ extern "C" int unomol_gpu_fock_rhf_noalloc(UnomolCtx* ctx, const double* dP, dou
     A.nshell = ctx->nshell;
     A.rys_compat = ctx->rys_mode == UNOMOL_RYS_REFERENCE;
     A.counters = nullptr;
-    A.mode = 0;
-    for (const ClassLaunch& L : ctx->launches) {
-        A.bps = ctx->d_bps + L.bp_begin;
-        A.prefix = ctx->d_prefix;
-        A.nbp = L.nbp;
-        A.nwork = L.nwork;
-        // the regular build's method selection: MD mode, runtime-L and MD classes included
-        CU(launch_class_kernel(ctx, L, false, false, A, s));
-        ++launches;
-    }
+    // the regular build's method selection: MD mode, runtime-L and MD classes included
+    for (size_t li = 0; li < ctx->launches.size(); ++li) CU(launch_plain_class(ctx, li, false, A, s, s, launches));
     CU(cudaEventRecord(ctx->ev[2], s));
     fold_packed<<<(unsigned)((np + 255) / 256), 256, 0, s>>>(T, dG, n);
     ++launches;

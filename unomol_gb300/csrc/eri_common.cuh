@@ -4,6 +4,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "df64.cuh"
+
 namespace ugb {
 
 constexpr int LMAX = 4;                 // largest shell angular momentum (g; Basis.hpp:222)
@@ -29,7 +31,9 @@ __host__ __device__ constexpr int cart_ly(int l, int c) {
 __host__ __device__ constexpr int cart_lz(int l, int c) { return l - cart_lx(l, c) - cart_ly(l, c); }
 
 // One primitive pair of a shell pair (a has the larger L after the swap of
-// TwoElectronInts.cpp:563-579); the kernels read it through the read-only path.
+// TwoElectronInts.cpp:563-579); the kernels read it through the read-only path.  The records of a shell
+// pair are in descending E (k_interleave_prims), so that a loop over them ends at the first one whose
+// prefactor can no longer pass the screen (plain FP64 build of 32 waters 21.8 -> 21.4 ms).
 struct __align__(16) PrimPair {
     double p;          // alpha_a + alpha_b
     double rp;         // 1 / p
@@ -48,6 +52,22 @@ struct __align__(16) PrimPair32 {
     float pad_;     // 48 bytes: three 16-byte loads
 };
 
+// The record in pairs of floats (48 bits, df64.cuh), for the quartets below SPLIT_CUT.  P is taken relative
+// to the middle of the molecule's box: only differences of centres are used, and their rounding follows the
+// distance to the origin.
+struct __align__(16) PrimPairDF {
+    df p, E;        // first 16-byte load: the prefactor screen
+    df Ecc, rp;
+    df P[3], PA[3];  // 80 bytes: five 16-byte loads
+};
+
+// Schwarz bound from which a quartet of the FP64 build is evaluated in FP64; below it, in pairs of floats
+// (fock_df64.cuh), whose error of about 2^-46 of the bound is then below 2e-15.  Chosen by the error of G
+// against the reference's fixtures, which stays what the all-FP64 build has up to a cut of 1/2 (a cut of 100,
+// every quartet in pairs of floats, doubles it on the three-water one), and by time (32 waters / n-decane
+// UHF): 1/128 24.7 / 5.3 ms, 1/32 23.2 / 4.6, 1/8 21.8 / 3.5, 1/2 20.4 / 3.4, 100 20.0 / 3.3.
+constexpr double SPLIT_CUT = 0.125;
+
 constexpr double SQRT_SRTERM = 5.914967172795613;  // sqrt(2 pi^{5/2})
 static_assert(SQRT_SRTERM * SQRT_SRTERM - SRTERM < 1e-13 && SRTERM - SQRT_SRTERM * SQRT_SRTERM < 1e-13, "sqrt of SRTERM");
 
@@ -63,10 +83,11 @@ struct ShellPair {
     double AB[3];          // A - B
     double q;              // Schwarz bound: max over functions of sqrt|(ab|ab)|
     int ish, jsh;          // shell indices (ish >= jsh)
-    int maxsh;             // max(ish, jsh)
     int pad;
+    float ABl[3];          // what A - B leaves over its FP32 copy, for the pairs-of-floats kernels
     float ABf[3];          // A - B and q in FP32, for the FP32 kernels (no FP64 work or conversion there)
     float qf;
+    int spare_[2];         // 112 bytes
 };
 
 // A rectangle (or triangle, when bra block == ket block) of quartets between two pair blocks,
@@ -86,6 +107,7 @@ struct FockArgs {
     const ShellPair* pairs;
     const PrimPair* prims;
     const PrimPair32* prims32;
+    const PrimPairDF* primsdf;
     const BlockPair* bps;
     const long long* prefix;    // concatenated staircase prefix sums
     int nbp;                    // block pairs of this launch
@@ -103,7 +125,8 @@ struct FockArgs {
     float thr_int32, prim_cut32, skip_cut32;  // the same cuts in FP32, for the FP32 kernels
     float fp32_cut32;           // mixed mode: a quartet with bound * max|P| of its blocks below this runs in FP32
     double fp32_cut;            // mixed mode: bound * max|P| below this -> FP32 part, else FP64 part
-    int mode;                   // 0 all quartets; 1 only "large" (FP64 part); 2 only "small" (FP32 part)
+    int mode;                   // 0 all quartets; 1 only "large" (FP64 part); 2 only "small" (FP32 part);
+                                // 3 / 4 the parts above / below SPLIT_CUT of an FP64 build
     int nshell;
     int rys_compat;             // reference-compatible two-root Rys regime (FP64 only)
     unsigned long long* counters;  // optional: primitive quartets past the prefactor cut, 32 slots per launch

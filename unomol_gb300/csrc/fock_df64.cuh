@@ -1,0 +1,328 @@
+// Shell-quartet integrals in pairs of floats (df64.cuh), for the quartets of the FP64 build whose Schwarz
+// bound lies below SPLIT_CUT.  The integrals of such a quartet are at most SPLIT_CUT, so the form's 2^-47
+// or so of the bound stays below half an ulp of an integral of order one, which every FP64 evaluation of
+// the larger quartets carries as well; the sum over the quartets, and with it G, keeps its error.  The
+// quartets above the cut are evaluated in FP64, and the density contraction and the accumulation are FP64
+// for all of them.
+//
+// What bounds it: the FP64 kernels keep the FP64 pipe (2 lanes per clock and SM) 88 % busy; the same
+// primitive quartet of (ps|ss) is about 65 FP64 instructions (1040 SM clocks per warp) or about 350 FP32
+// ones (88 clocks at full issue).  Here issue is 50-60 % active, the L1 data pipe 50-60 % and the FP64 pipe
+// (the density contraction) 17-33 %, with the loads the leading stall.  One build, GB300: 32 waters 6-31G
+// 78.5 -> 22.3 ms, n-decane cation UHF 12.1 -> 3.5 ms (with the group kernels below).
+// Measured beside it: look-ahead for the next surviving primitive quartet (as the FP64 kernels) instead of
+// plain loops, kept for la+lb+lc+ld = 2 only ((ps|ps) 3.9 against 4.2 ms, (ps|ss) 7.6 against 6.9); 64
+// registers for (ss|ss) and (ps|ss) (25.3 -> 24.0 ms for the build).
+#pragma once
+#include <type_traits>
+
+#include "df64.cuh"
+#include "fock_kernels.cuh"
+
+
+namespace ugb {
+
+// Rows of the root tables: 8 leading parts (highest power first), then the 8 remainders.
+constexpr int DF_STRIDE = 16;
+constexpr int DF_ROWS_END = rys_off(RYS_NMAX + 1, DF_STRIDE, RYS_H);
+// a second two-root block whose intervals in (15, 40] hold the reference's own large-T form
+constexpr int DF_COMPAT2 = DF_ROWS_END;
+constexpr int DF_HERMITE = DF_COMPAT2 + rys_off(3, DF_STRIDE, RYS_H) - rys_off(2, DF_STRIDE, RYS_H);
+constexpr int DF_TABLE_LEN = DF_HERMITE + 100;  // x[5][5] (h, l), w[5][5] (h, l)
+static_assert(RYS_DEG == 7 && RYS_H == 0.25, "the double-float table rows and the index below");
+
+// One table polynomial at y = yh + yl.  Coefficient k is about 0.125^k / k! of the first, so the three
+// highest powers need only floats: their rounding lies below 2^-50 of the value.
+__device__ __forceinline__ df df_poly(const float* __restrict__ c, float yh, float yl) {
+    float h[8], l[8];
+    load_row(c, h);
+    load_row(c + 8, l);
+    float v = __fmaf_rn(h[0], yh, h[1]);
+    // power 5: its own leading part, everything above it in the remainder
+    df r = {h[2], __fmaf_rn(v, yh, l[2])};
+#pragma unroll
+    for (int k = 3; k < 8; ++k) {
+        const float p = __fmul_rn(r.h, yh);
+        float e = __fmaf_rn(r.h, yh, -p);
+        e = __fmaf_rn(r.l, yh, e);
+        e = __fmaf_rn(r.h, yl, e);
+        const df t = df_add({h[k], l[k]}, {p, e});
+        r = t;
+    }
+    return r;
+}
+
+// Rys nodes and weights in double-float; rs_T etc. as rys_roots.  compat: the two-root block with the
+// reference's form in 15 < T <= 40.
+template <int NR, bool NEED_X>
+__device__ __forceinline__ void df_roots(df T, const float* __restrict__ tab, bool compat, df* x, df* w) {
+    constexpr float TMAX = float(rys_tmax(NR));
+    if (T.h < TMAX) {
+        const float f = 4.0f * T.h;
+        int k;
+        const float* blk = tab + rys_off(NR, DF_STRIDE, RYS_H);
+        if constexpr (NR == 2) {
+            // intervals (k H, (k + 1) H]: the reference's form starts above T = 15 and ends at T = 40
+            const float c = ceilf(f);
+            k = (int)c - ((c == f && T.l > 0.f) ? 0 : 1);
+            k = max(k, 0);
+            if (compat) blk = tab + DF_COMPAT2;
+        } else {
+            k = max((int)f, 0);
+        }
+        // y = 2 (T / H - k) - 1 = 8 T - (2 k + 1); the leading part rounds only below T = 1/8
+        const float T8 = 8.0f * T.h, m = float(2 * k + 1), yh = __fsub_rn(T8, m);
+        const float yl = __fmaf_rn(8.0f, T.l, __fsub_rn(T8, __fadd_rn(yh, m)));
+        blk += k * (2 * NR * DF_STRIDE);
+#pragma unroll
+        for (int i = 0; i < NR; ++i) {
+            if (NEED_X) x[i] = df_poly(blk + 2 * i * DF_STRIDE, yh, yl);
+            w[i] = df_poly(blk + (2 * i + 1) * DF_STRIDE, yh, yl);
+        }
+    } else {
+        const float2* herm = reinterpret_cast<const float2*>(tab + DF_HERMITE);
+        const df s = df_rsqrt(T);
+        const df r = df_sqr(s);
+#pragma unroll
+        for (int i = 0; i < NR; ++i) {
+            const float2 hx = __ldg(herm + (NR - 1) * 5 + i), hw = __ldg(herm + 25 + (NR - 1) * 5 + i);
+            if (NEED_X) x[i] = df_mul({hx.x, hx.y}, r);
+            w[i] = df_mul({hw.x, hw.y}, s);
+        }
+    }
+}
+
+// rys_axis (fock_kernels.cuh) in double-float.  UNIT: the axis starts from 1 (its factor sits on the z
+// axis), so products with element (0, 0) fall away.
+template <int LA, int LB, int LC, int LD, bool UNIT>
+__device__ __forceinline__ void df_axis(df g00, df C, df Cp, df B00, df B1, df B1p, df AB, df CD,
+                                        df (&I)[(LA + 1) * (LB + 1) * (LC + 1) * (LD + 1)]) {
+    constexpr int L12 = LA + LB, L34 = LC + LD;
+    // a x + y with x element (ix) of the recurrence, which is 1 for UNIT at index 0
+    auto mad = [](bool one, df a, df x, df y) { return (UNIT && one) ? df_add(y, a) : df_fma(a, x, y); };
+    auto prod = [](bool one, df a, df x) { return (UNIT && one) ? a : df_mul(a, x); };
+    df G[L12 + 1][L34 + 1];
+    G[0][0] = g00;
+    if constexpr (L12 > 0) G[1][0] = prod(true, C, g00);
+#pragma unroll
+    for (int i = 1; i < L12; ++i) {
+        const df b = i == 1 ? B1 : df_mulf(B1, float(i));
+        G[i + 1][0] = mad(i == 1, b, G[i - 1][0], df_mul(C, G[i][0]));
+    }
+#pragma unroll
+    for (int j = 0; j < L34; ++j) {
+#pragma unroll
+        for (int i = 0; i <= L12; ++i) {
+            df v = prod(i == 0 && j == 0, Cp, G[i][j]);
+            if (j > 0) v = mad(i == 0 && j == 1, j == 1 ? B1p : df_mulf(B1p, float(j)), G[i][j - 1], v);
+            if (i > 0) v = mad(i == 1 && j == 0, i == 1 ? B00 : df_mulf(B00, float(i)), G[i - 1][j], v);
+            G[i][j + 1] = v;
+        }
+    }
+    df X[LB + 1][L12 + 1][L34 + 1];
+#pragma unroll
+    for (int a = 0; a <= L12; ++a)
+#pragma unroll
+        for (int j = 0; j <= L34; ++j) X[0][a][j] = G[a][j];
+#pragma unroll
+    for (int b = 1; b <= LB; ++b)
+#pragma unroll
+        for (int a = 0; a <= L12 - b; ++a)
+#pragma unroll
+            for (int j = 0; j <= L34; ++j)
+                X[b][a][j] = mad(b == 1 && a == 0 && j == 0, AB, X[b - 1][a][j], X[b - 1][a + 1][j]);
+#pragma unroll
+    for (int a = 0; a <= LA; ++a)
+#pragma unroll
+        for (int b = 0; b <= LB; ++b) {
+            df Y[LD + 1][L34 + 1];
+#pragma unroll
+            for (int c = 0; c <= L34; ++c) Y[0][c] = X[b][a][c];
+#pragma unroll
+            for (int d = 1; d <= LD; ++d)
+#pragma unroll
+                for (int c = 0; c <= L34 - d; ++c)
+                    Y[d][c] = mad(a == 0 && b == 0 && c == 0 && d == 1, CD, Y[d - 1][c], Y[d - 1][c + 1]);
+#pragma unroll
+            for (int c = 0; c <= LC; ++c)
+#pragma unroll
+                for (int d = 0; d <= LD; ++d) I[((a * (LB + 1) + b) * (LC + 1) + c) * (LD + 1) + d] = Y[d][c];
+        }
+}
+
+// FP32 -> FP64 through the integer pipe as f32_to_f64, with infinities and NaN kept
+__device__ __forceinline__ double df_to_f64(df a) {
+    auto cvt = [](float f) {
+        const unsigned u = __float_as_uint(f);
+        const unsigned e = (u >> 23) & 0xffu;
+        const unsigned ex = e == 0xffu ? 0x7ffu : e + 896u;
+        const unsigned hi = (u & 0x80000000u) | (e ? ((ex << 20) | ((u >> 3) & 0xfffffu)) : 0u);
+        return __hiloint2double((int)hi, (int)(e ? (u << 29) : 0u));
+    };
+    return cvt(a.h) + cvt(a.l);
+}
+
+// Contracted integrals of one shell quartet as shell_quartet_eri<..., double>, in double-float: the same
+// primitive quartets (prefactor screen on floats, decided in double-float within 0.1 % of the cut).
+template <int LA, int LB, int LC, int LD>
+__device__ __forceinline__ void shell_quartet_df64(const ShellPair& bra, const ShellPair& ket,
+                                                   const PrimPairDF* __restrict__ prims, const float* __restrict__ tab,
+                                                   float prim_cut32, bool compat, df (&acc)[QClass<LA, LB, LC, LD>::NF],
+                                                   unsigned* npass) {
+    using Q = QClass<LA, LB, LC, LD>;
+    constexpr int NR = Q::NR;
+    constexpr int L12 = LA + LB, L34 = LC + LD;
+#pragma unroll
+    for (int f = 0; f < Q::NF; ++f) acc[f] = {0.f, 0.f};
+    const PrimPairDF* pb = prims + bra.prim_begin;
+    const PrimPairDF* pk = prims + ket.prim_begin;
+    const int nb = bra.nprim, nk = ket.nprim, sb = bra.prim_stride, sk = ket.prim_stride;
+    const float lo32 = prim_cut32 * 0.999f, hi32 = prim_cut32 * 1.001f;
+    // the prefactor screen on floats; in the band around the cut on all 48 bits (TwoElectronInts.cpp:478-479)
+    auto passes = [&](const df& bp_p, const df& bp_E, const df& kp_p, const df& kp_E) {
+        const float v32 = float(SRTERM) * bp_E.h * kp_E.h * rsqrtf(bp_p.h + kp_p.h);
+        if (v32 < lo32) return false;
+        if (v32 <= hi32) {
+            const float sh = float(SRTERM), sl = float(SRTERM - double(float(SRTERM)));
+            const float ch = float(PRIM_CUT), cl = float(PRIM_CUT - double(float(PRIM_CUT)));
+            const df v = df_mul(df_mul({sh, sl}, df_mul(bp_E, kp_E)), df_rsqrt(df_add(bp_p, kp_p)));
+            if (!(__fadd_rn(__fsub_rn(v.h, ch), __fsub_rn(v.l, cl)) > 0.f)) return false;
+        }
+        return true;
+    };
+    auto primitive = [&](const PrimPairDF& bp, const PrimPairDF& kp) {
+        if (npass) ++*npass;
+        const df rs = df_rsqrt(df_add(bp.p, kp.p));
+        const df sr = df_mul(df_mul(bp.Ecc, kp.Ecc), rs);
+        const df rpq = df_sqr(rs);
+        const df PQx = df_sub(bp.P[0], kp.P[0]), PQy = df_sub(bp.P[1], kp.P[1]), PQz = df_sub(bp.P[2], kp.P[2]);
+        const df R2 = df_add(df_add(df_sqr(PQx), df_sqr(PQy)), df_sqr(PQz));
+        const df T = df_mul(df_mul(df_mul(bp.p, kp.p), rpq), R2);
+        df x[NR], w[NR];
+        df_roots<NR, L12 + L34 != 0>(T, tab, compat, x, w);
+        if constexpr (L12 + L34 == 0) {
+            acc[0] = df_fma(w[0], sr, acc[0]);
+        } else {
+#pragma unroll
+            for (int r = 0; r < NR; ++r) {
+                const df fff = df_mul(x[r], rpq);  // t^2 / (p + q)   (Rys.hpp:126-129)
+                const df zero = {0.f, 0.f};
+                const df qf = L12 > 0 ? df_mul(kp.p, fff) : zero, pf = L34 > 0 ? df_mul(bp.p, fff) : zero;
+                const df B00 = (L12 > 0 && L34 > 0) ? df_half(fff) : zero;
+                // (1/2 - q B00) / p = (1 - q t^2 / (p + q)) / 2 p
+                const df B1 = L12 > 1 ? df_half(df_mul(df_rsubf(1.f, qf), bp.rp)) : zero;
+                const df B1p = L34 > 1 ? df_half(df_mul(df_rsubf(1.f, pf), kp.rp)) : zero;
+                df Ix[Q::NI], Iy[Q::NI], Iz[Q::NI];
+                const df nqf = df_neg(qf);
+                auto axis = [&](int k, const df& PQ, auto unit, df g, df(&I)[Q::NI]) {
+                    const df C = L12 > 0 ? df_fma(nqf, PQ, bp.PA[k]) : zero, Cp = L34 > 0 ? df_fma(pf, PQ, kp.PA[k]) : zero;
+                    const df AB = LB > 0 ? df{bra.ABf[k], bra.ABl[k]} : zero, CD = LD > 0 ? df{ket.ABf[k], ket.ABl[k]} : zero;
+                    df_axis<LA, LB, LC, LD, decltype(unit)::value>(g, C, Cp, B00, B1, B1p, AB, CD, I);
+                };
+                axis(0, PQx, std::true_type{}, df{1.f, 0.f}, Ix);
+                axis(1, PQy, std::true_type{}, df{1.f, 0.f}, Iy);
+                axis(2, PQz, std::false_type{}, df_mul(w[r], sr), Iz);
+#pragma unroll
+                for (int ia = 0; ia < Q::NA; ++ia)
+#pragma unroll
+                    for (int ibb = 0; ibb < Q::NB; ++ibb)
+#pragma unroll
+                        for (int ic = 0; ic < Q::NC; ++ic)
+#pragma unroll
+                            for (int id = 0; id < Q::ND; ++id) {
+                                const int f = ((ia * Q::NB + ibb) * Q::NC + ic) * Q::ND + id;
+                                const int jx = Q::iidx(cart_lx(LA, ia), cart_lx(LB, ibb), cart_lx(LC, ic), cart_lx(LD, id));
+                                const int jy = Q::iidx(cart_ly(LA, ia), cart_ly(LB, ibb), cart_ly(LC, ic), cart_ly(LD, id));
+                                const int jz = Q::iidx(cart_lz(LA, ia), cart_lz(LB, ibb), cart_lz(LC, ic), cart_lz(LD, id));
+                                // element 0 of the x and y axes is 1
+                                if (jx == 0 && jy == 0) acc[f] = df_add(acc[f], Iz[jz]);
+                                else if (jx == 0) acc[f] = df_fma(Iy[jy], Iz[jz], acc[f]);
+                                else if (jy == 0) acc[f] = df_fma(Ix[jx], Iz[jz], acc[f]);
+                                else acc[f] = df_fma(df_mul(Ix[jx], Iy[jy]), Iz[jz], acc[f]);
+                            }
+            }
+        }
+    };
+    if constexpr (L12 + L34 == 2) {
+        int ib = 0, ik = 0, cb = -1;
+        float rowf = 0.f;  // bound of SRTERM E_ab / sqrt(p + q) over the kets
+        PrimPairDF bp = pb[0];
+        for (;;) {
+            PrimPairDF kp;
+            bool found = false;
+            while (ib < nb) {
+                if (ib != cb) {
+                    bp = pb[ib * sb];
+                    cb = ib;
+                    rowf = float(SRTERM) * bp.E.h * rsqrtf(bp.p.h);
+                }
+                kp = pk[ik * sk];
+                if (rowf * kp.E.h < lo32) {  // E_cd descends: no later ket primitive passes either
+                    ik = 0;
+                    ++ib;
+                    continue;
+                }
+                if (++ik == nk) {
+                    ik = 0;
+                    ++ib;
+                }
+                if (!passes(bp.p, bp.E, kp.p, kp.E)) continue;
+                found = true;
+                break;
+            }
+            if (!found) break;
+            primitive(bp, kp);
+        }
+    } else {
+        for (int ik = 0; ik < nk; ++ik) {
+            const PrimPairDF kp = pk[ik * sk];
+            const float colf = float(SRTERM) * kp.E.h * rsqrtf(kp.p.h);
+            for (int ib = 0; ib < nb; ++ib) {
+                const PrimPairDF bp = pb[ib * sb];
+                if (colf * bp.E.h < lo32) break;  // E_ab descends: no later bra primitive passes either
+                if (!passes(bp.p, bp.E, kp.p, kp.E)) continue;
+                primitive(bp, kp);
+            }
+        }
+    }
+}
+
+// The quartets below SPLIT_CUT of one class: integrals in double-float, density contraction and scatter in
+// FP64 as the FP64 kernels.
+template <int LA, int LB, int LC, int LD, bool UHF>
+__global__ void __launch_bounds__(128, LA + LB + LC + LD <= 1 ? 8 : 1) fock_jk_df64(const FockArgs A, const NormTable nt, const float* __restrict__ tab) {
+    using Q = QClass<LA, LB, LC, LD>;
+    int bi, ki;
+    if (!decode_work_warp<true>(A, (long long)blockIdx.x * blockDim.x + threadIdx.x, bi, ki)) return;
+    const ShellPair bra = A.pairs[bi];
+    const ShellPair ket = A.pairs[ki];
+    unsigned npass = 0;
+    double v[Q::NF];
+    {
+        df acc[Q::NF];
+        shell_quartet_df64<LA, LB, LC, LD>(bra, ket, A.primsdf, tab, A.prim_cut32, A.rys_compat != 0, acc,
+                                           A.counters ? &npass : nullptr);
+#pragma unroll
+        for (int f = 0; f < Q::NF; ++f) v[f] = df_to_f64(acc[f]);
+    }
+    digest_jk<LA, LB, LC, LD, UHF, double>(A, bra, ket, bi == ki, v, nt);
+    if (A.counters) count_flush(A, npass);
+}
+
+// FP64 integrals with NP lanes per shell quartet, each summing every NP-th primitive quartet: where a launch
+// holds few quartets, one lane each leaves the GPU idle behind a serial chain of primitive quartets (water in
+// STO-3G, 81 of them per quartet: 1.36 -> 0.17 ms per build with a warp each).  DYN: the quartets of a split
+// list (those at or above SPLIT_CUT: few, and the costliest of the build); otherwise every quartet of the class.
+template <int LA, int LB, int LC, int LD, bool UHF, int NP, bool DYN>
+__global__ void __launch_bounds__(128) fock_jk_fp64_group(const FockArgs A, const NormTable nt, const double* __restrict__ rys) {
+    const int lane = threadIdx.x & 31, sub = lane / NP, part = lane % NP;
+    const unsigned gmask = NP == 32 ? 0xffffffffu : ((1u << (NP & 31)) - 1u) << (sub * NP);
+    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    int bi, ki;
+    if (!decode_warp_items<DYN>(A, warp * (32 / NP), sub, bi, ki)) return;  // uniform over a group
+    const ShellPair bra = A.pairs[bi];
+    const ShellPair ket = A.pairs[ki];
+    quartet_item_group<LA, LB, LC, LD, UHF, double, NP>(A, nt, rys, bra, ket, bi == ki, part, gmask);
+}
+
+}  // namespace ugb

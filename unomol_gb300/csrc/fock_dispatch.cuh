@@ -2,6 +2,8 @@
 // quartet classes are (bra class >= ket class).  One translation unit per arithmetic type
 // instantiates all of them (fock_fp64.cu, fock_fp32.cu).
 #pragma once
+#include <vector>
+
 #include "eri_common.cuh"
 
 namespace ugb {
@@ -28,6 +30,15 @@ cudaError_t launch_fock_fp64_part(int bc, int kc, bool uhf, const FockArgs& A64,
                                   const double* rys64, const float* rys32, int grid, cudaStream_t stream);
 cudaError_t launch_schwarz(int pc, const ShellPair* pairs, const PrimPair* prims, int begin, int count,
                            const NormTable& nt, const double* rys, double* q_out, cudaStream_t stream);
+
+// The quartets below SPLIT_CUT of one class in pairs of floats (fock_df64.cuh), `items` of its split list.
+cudaError_t launch_fock_df64(int bc, int kc, bool uhf, const FockArgs& A, long long items, const NormTable& nt,
+                             const float* tab, cudaStream_t stream);
+// One class in FP64 with `lanes` (4 or 32) lanes per quartet: `items` of a split list (dyn) or of the whole class.
+cudaError_t launch_fock_fp64_group(int bc, int kc, bool uhf, const FockArgs& A, long long items, bool dyn, int lanes,
+                                   const NormTable& nt, const double* rys, cudaStream_t stream);
+// Both take the classes that fock_mixed_fused accepts.  The root tables of the first:
+std::vector<float> df_rys_tables();
 
 // Runtime-L Rys kernel (classes with f or g shells and la+lb+lc+ld <= 8), FP64 or FP32.
 cudaError_t launch_fock_generic(int la, int lb, int lc, int ld, bool uhf, bool fp32, const FockArgs& A,

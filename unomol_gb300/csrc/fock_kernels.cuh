@@ -77,6 +77,17 @@ __device__ __forceinline__ double f32_to_f64(float f) {
     const unsigned lo = e ? (u << 29) : 0u;
     return __hiloint2double((int)hi, (int)lo);
 }
+// v 2^n for a normal v whose result stays normal (the integrals past the storage cut)
+__device__ __forceinline__ double scale_pow2(double v, int n) {
+    return __hiloint2double(__double2hiint(v) + n * (1 << 20), __double2loint(v));
+}
+__device__ __forceinline__ float scale_pow2(float v, int n) { return __int_as_float(__float_as_int(v) + n * (1 << 23)); }
+// v 2^n, n >= 0, for any v (zero, subnormal, infinite and NaN values by a product)
+__device__ __forceinline__ double scale_sum(double v, int n) {
+    const int hi = __double2hiint(v), e = (hi >> 20) & 0x7ff;
+    return (unsigned)(e - 1) < 2046u - 8u ? scale_pow2(v, n) : v * double(1 << n);
+}
+__device__ __forceinline__ float scale_sum(float v, int n) { return v * float(1 << n); }
 __device__ __forceinline__ double to_f64(double v) { return v; }
 __device__ __forceinline__ double to_f64(float v) { return f32_to_f64(v); }
 
@@ -405,6 +416,7 @@ __device__ __forceinline__ void shell_quartet_eri(const ShellPair& bra, const Sh
         // quartets were screened out do not sit idle through another lane's FP64 work.
         const float lo32 = prim_cut32 * 0.999f, hi32 = prim_cut32 * 1.001f;
         int ib = 0, ik = 0, cb = -1;
+        float rowf = 0.f;  // bound of SRTERM E_ab / sqrt(p + q) over the kets
         PP bp = pb[0];
         for (;;) {
             PP kp;
@@ -414,8 +426,14 @@ __device__ __forceinline__ void shell_quartet_eri(const ShellPair& bra, const Sh
                 if (ib != cb) {
                     bp = pb[ib * sb];  // whole 16-byte-aligned records: vector loads
                     cb = ib;
+                    rowf = float(SRTERM) * bp.Ef * rsqrtf(bp.pf);
                 }
                 kp = pk[ik * sk];
+                if (rowf * kp.Ef < lo32) {  // E_cd descends: no later ket primitive passes either
+                    ik = 0;
+                    ++ib;
+                    continue;
+                }
                 if (++ik == nk) {
                     ik = 0;
                     ++ib;
@@ -537,7 +555,7 @@ __device__ __forceinline__ bool decode_warp_items(const FockArgs& A, long long g
     while (a + 1 < bp.bra_count && pre[a + 1] <= w) ++a;
     bra_idx = bp.bra_begin + a;
     int j = (int)(w - pre[a]);
-    if (DYN && A.mode == 2) j += A.dyn_mseg[bp.prefix_off + a];
+    if (DYN && (A.mode & 1) == 0) j += A.dyn_mseg[bp.prefix_off + a];
     ket_idx = bp.ket_begin + j;
     return true;
 }
@@ -592,10 +610,9 @@ __device__ __forceinline__ void digest_jk(const FockArgs& A, const ShellPair& br
     }
     double* __restrict__ Ta = A.Ta + base;
     double* __restrict__ Tb = UHF ? A.Tb + base : nullptr;
-    R deg = R(1);
-    if (bra.same) deg *= R(0.5);
-    if (ket.same) deg *= R(0.5);
-    if (same_pair) deg *= R(0.5);
+    // The degeneracy factor 1/2 per coincidence and the 4 (2) of the Coulomb sums are powers of two: applied
+    // to the exponent fields, on the integer pipe (per (ss|ss) quartet 18 -> 7 FP64 instructions).
+    const int ndeg = (bra.same != 0) + (ket.same != 0) + (same_pair ? 1 : 0);
     const R* __restrict__ Pa;
     const R* __restrict__ Pb;
     if constexpr (sizeof(R) == 8) {
@@ -605,7 +622,7 @@ __device__ __forceinline__ void digest_jk(const FockArgs& A, const ShellPair& br
         Pa = reinterpret_cast<const R*>(A.Pa32) + base;
         Pb = UHF ? reinterpret_cast<const R*>(A.Pb32) + base : nullptr;
     }
-    const R jf = UHF ? R(2) : R(4);
+    constexpr int JEXP = UHF ? 1 : 2;
     R thr;
     if constexpr (sizeof(R) == 4) thr = A.thr_int32;
     else thr = A.thr_int;
@@ -645,36 +662,37 @@ __device__ __forceinline__ void digest_jk(const FockArgs& A, const ShellPair& br
                         else v *= nt.v[LA][ia] * nt.v[LB][ib] * nt.v[LC][ic] * nt.v[LD][id];
                     }
                     if (!above_cut(v, thr)) continue;  // TwoElectronInts.cpp:668
+                    v = scale_pow2(v, -ndeg);
                     R Pcd = __ldg(Pa + c * N + d);
                     if constexpr (UHF) Pcd += __ldg(Pb + c * N + d);
                     jab = fma(v, Pcd, jab);
                     jcd[ic * Q::ND + id] = fma(v, Pab, jcd[ic * Q::ND + id]);
-                    kac[ic] = fma(v, __ldg(Pa + b * N + d), kac[ic]);
-                    kad[id] = fma(v, __ldg(Pa + b * N + c), kad[id]);
-                    kbc[ib * Q::NC + ic] = fma(v, __ldg(Pa + a * N + d), kbc[ib * Q::NC + ic]);
-                    kbd[ib * Q::ND + id] = fma(v, __ldg(Pa + a * N + c), kbd[ib * Q::ND + id]);
+                    kac[ic] = fma(-v, __ldg(Pa + b * N + d), kac[ic]);
+                    kad[id] = fma(-v, __ldg(Pa + b * N + c), kad[id]);
+                    kbc[ib * Q::NC + ic] = fma(-v, __ldg(Pa + a * N + d), kbc[ib * Q::NC + ic]);
+                    kbd[ib * Q::ND + id] = fma(-v, __ldg(Pa + a * N + c), kbd[ib * Q::ND + id]);
                     if constexpr (UHF) {
-                        kacB[ic] = fma(v, __ldg(Pb + b * N + d), kacB[ic]);
-                        kadB[id] = fma(v, __ldg(Pb + b * N + c), kadB[id]);
-                        kbcB[ib * Q::NC + ic] = fma(v, __ldg(Pb + a * N + d), kbcB[ib * Q::NC + ic]);
-                        kbdB[ib * Q::ND + id] = fma(v, __ldg(Pb + a * N + c), kbdB[ib * Q::ND + id]);
+                        kacB[ic] = fma(-v, __ldg(Pb + b * N + d), kacB[ic]);
+                        kadB[id] = fma(-v, __ldg(Pb + b * N + c), kadB[id]);
+                        kbcB[ib * Q::NC + ic] = fma(-v, __ldg(Pb + a * N + d), kbcB[ib * Q::NC + ic]);
+                        kbdB[ib * Q::ND + id] = fma(-v, __ldg(Pb + a * N + c), kbdB[ib * Q::ND + id]);
                     }
                 }
             }
-            add_bra_sum<R>(Ta + a * N + b, jf * deg * jab);
-            if constexpr (UHF) add_bra_sum<R>(Tb + a * N + b, jf * deg * jab);
+            add_bra_sum<R>(Ta + a * N + b, scale_sum(jab, JEXP));
+            if constexpr (UHF) add_bra_sum<R>(Tb + a * N + b, scale_sum(jab, JEXP));
         }
 #pragma unroll
         for (int ic = 0; ic < Q::NC; ++ic) {
             const int c = ket.a_off + ic;
-            atomicAdd(Ta +a * N + c, to_f64(-deg * kac[ic]));
-            if constexpr (UHF) atomicAdd(Tb +a * N + c, to_f64(-deg * kacB[ic]));
+            atomicAdd(Ta +a * N + c, to_f64(kac[ic]));
+            if constexpr (UHF) atomicAdd(Tb +a * N + c, to_f64(kacB[ic]));
         }
 #pragma unroll
         for (int id = 0; id < Q::ND; ++id) {
             const int d = ket.b_off + id;
-            atomicAdd(Ta +a * N + d, to_f64(-deg * kad[id]));
-            if constexpr (UHF) atomicAdd(Tb +a * N + d, to_f64(-deg * kadB[id]));
+            atomicAdd(Ta +a * N + d, to_f64(kad[id]));
+            if constexpr (UHF) atomicAdd(Tb +a * N + d, to_f64(kadB[id]));
         }
     }
 #pragma unroll
@@ -682,7 +700,7 @@ __device__ __forceinline__ void digest_jk(const FockArgs& A, const ShellPair& br
 #pragma unroll
         for (int id = 0; id < Q::ND; ++id) {
             const int c = ket.a_off + ic, d = ket.b_off + id;
-            const double j = to_f64(jf * deg * jcd[ic * Q::ND + id]);
+            const double j = to_f64(scale_sum(jcd[ic * Q::ND + id], JEXP));
             atomicAdd(Ta +c * N + d, j);
             if constexpr (UHF) atomicAdd(Tb +c * N + d, j);
         }
@@ -692,14 +710,14 @@ __device__ __forceinline__ void digest_jk(const FockArgs& A, const ShellPair& br
 #pragma unroll
         for (int ic = 0; ic < Q::NC; ++ic) {
             const int c = ket.a_off + ic;
-            atomicAdd(Ta +b * N + c, to_f64(-deg * kbc[ib * Q::NC + ic]));
-            if constexpr (UHF) atomicAdd(Tb +b * N + c, to_f64(-deg * kbcB[ib * Q::NC + ic]));
+            atomicAdd(Ta +b * N + c, to_f64(kbc[ib * Q::NC + ic]));
+            if constexpr (UHF) atomicAdd(Tb +b * N + c, to_f64(kbcB[ib * Q::NC + ic]));
         }
 #pragma unroll
         for (int id = 0; id < Q::ND; ++id) {
             const int d = ket.b_off + id;
-            atomicAdd(Ta +b * N + d, to_f64(-deg * kbd[ib * Q::ND + id]));
-            if constexpr (UHF) atomicAdd(Tb +b * N + d, to_f64(-deg * kbdB[ib * Q::ND + id]));
+            atomicAdd(Ta +b * N + d, to_f64(kbd[ib * Q::ND + id]));
+            if constexpr (UHF) atomicAdd(Tb +b * N + d, to_f64(kbdB[ib * Q::ND + id]));
         }
     }
 }

@@ -52,7 +52,6 @@ __global__ void k_build_pairs(const ShellsDev sh, int npairs, const int* __restr
     ShellPair sp{};
     sp.ish = ish;
     sp.jsh = jsh;
-    sp.maxsh = ish;
     sp.prim_stride = 1;  // canonical layout until the pairs are interleaved by block
     sp.same = ish == jsh;
     sp.la = sh.sl[a];
@@ -64,6 +63,7 @@ __global__ void k_build_pairs(const ShellsDev sh, int npairs, const int* __restr
     for (int k = 0; k < 3; ++k) {
         sp.AB[k] = __dsub_rn(A[k], B[k]);
         sp.ABf[k] = (float)sp.AB[k];
+        sp.ABl[k] = (float)(sp.AB[k] - (double)sp.ABf[k]);
     }
     const double ab2 = __dadd_rn(__dadd_rn(__dmul_rn(sp.AB[0], sp.AB[0]), __dmul_rn(sp.AB[1], sp.AB[1])),
                                  __dmul_rn(sp.AB[2], sp.AB[2]));
@@ -155,31 +155,61 @@ __global__ void k_row_bp(const BlockPair* __restrict__ bps, int* __restrict__ ro
     for (int i = threadIdx.x; i < bp.bra_count; i += blockDim.x) row_bp[bp.prefix_off + i] = (int)blockIdx.x;
 }
 
+__device__ __forceinline__ df split_df(double v) {
+    const float h = (float)v;
+    return {h, (float)(v - (double)h)};
+}
+
 // Final layout of the primitive pairs: block b (pairs bbegin[b] .. + bcount[b], all with the same
 // primitive-pair count) owns records bprim[b] .. + bcount[b] * nprim, and primitive ik of its j-th pair
 // sits at bprim[b] + ik * bcount[b] + j, so that the lanes of a warp, which hold consecutive pairs of a
-// block, read adjacent records.  One thread per pair; src is the canonical layout.
+// block, read adjacent records.  src is the canonical layout, which dst32 keeps within a pair; dst has a
+// pair's records in descending E (equal ones in canonical order), which puts the primitive quartets past the prefactor screen first, at
+// the same places for the neighbouring pairs of a warp.  dstdf: the same records in pairs of floats, P
+// relative to `org`.  One warp per pair, each lane finding the rank of its records.
 __global__ void k_interleave_prims(ShellPair* __restrict__ pairs, int n, const int* __restrict__ bbegin,
                                    const int* __restrict__ bcount, const long long* __restrict__ bprim, int nb,
                                    const PrimPair* __restrict__ src, const PrimPair32* __restrict__ src32,
-                                   PrimPair* __restrict__ dst, PrimPair32* __restrict__ dst32) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
+                                   PrimPair* __restrict__ dst, PrimPair32* __restrict__ dst32,
+                                   PrimPairDF* __restrict__ dstdf, double3 org) {
+    const int k = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (k >= n) return;  // whole warps
     int lo = 0, hi = nb - 1;  // the block: last with bbegin <= k
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
         if (bbegin[mid] <= k) lo = mid; else hi = mid - 1;
     }
     const int j = k - bbegin[lo], cnt = bcount[lo];
-    ShellPair sp = pairs[k];
+    const int begin = pairs[k].prim_begin, np = pairs[k].nprim;
     const long long first = bprim[lo] + j;
-    for (int ik = 0; ik < sp.nprim; ++ik) {
-        dst[first + (long long)ik * cnt] = src[sp.prim_begin + ik];
-        dst32[first + (long long)ik * cnt] = src32[sp.prim_begin + ik];
+    for (int ik = lane; ik < np; ik += 32) {
+        const PrimPair pp = src[begin + ik];
+        // E >= 0 orders as its bit pattern (a NaN, of coordinates that are none, too: ranks stay distinct)
+        const long long key = __double_as_longlong(pp.E);
+        int rank = 0;
+        for (int m = 0; m < np; ++m) {
+            const long long other = __double_as_longlong(src[begin + m].E);
+            rank += other > key || (other == key && m < ik);
+        }
+        const long long at = first + (long long)rank * cnt;
+        dst[at] = pp;
+        dst32[first + (long long)ik * cnt] = src32[begin + ik];
+        PrimPairDF d;
+        d.p = split_df(pp.p);
+        d.E = split_df(pp.E);
+        d.Ecc = split_df(pp.Ecc);
+        d.rp = split_df(pp.rp);
+        d.P[0] = split_df(pp.P[0] - org.x);
+        d.P[1] = split_df(pp.P[1] - org.y);
+        d.P[2] = split_df(pp.P[2] - org.z);
+        for (int x = 0; x < 3; ++x) d.PA[x] = split_df(pp.PA[x]);
+        dstdf[at] = d;
     }
-    sp.prim_begin = (int)first;
-    sp.prim_stride = cnt;
-    pairs[k] = sp;
+    __syncwarp();
+    if (lane == 0) {
+        pairs[k].prim_begin = (int)first;
+        pairs[k].prim_stride = cnt;
+    }
 }
 
 __global__ void k_offset_pairs(ShellPair* __restrict__ pairs, int n, int prim0, int mol) {
@@ -233,9 +263,10 @@ cudaError_t setup_row_bp(const BlockPair* bps, int nbp, int* row_bp, cudaStream_
 
 cudaError_t setup_interleave_prims(ShellPair* pairs, int n, const int* bbegin, const int* bcount, const long long* bprim,
                                    int nb, const PrimPair* src, const PrimPair32* src32, PrimPair* dst, PrimPair32* dst32,
-                                   cudaStream_t s) {
+                                   PrimPairDF* dstdf, const double* origin, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    k_interleave_prims<<<blocks_for(n, 128), 128, 0, s>>>(pairs, n, bbegin, bcount, bprim, nb, src, src32, dst, dst32);
+    k_interleave_prims<<<blocks_for(32ll * n, 128), 128, 0, s>>>(pairs, n, bbegin, bcount, bprim, nb, src, src32, dst, dst32,
+                                                         dstdf, make_double3(origin[0], origin[1], origin[2]));
     return cudaGetLastError();
 }
 
