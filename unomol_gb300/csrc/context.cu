@@ -665,7 +665,7 @@ cudaError_t launch_plain_class(const UnomolCtx* ctx, size_t li, bool uhf, FockAr
     A.nwork = L.nwork;
     A.mode = 0;
     const int lsum = pc_la(L.bc) + pc_lb(L.bc) + pc_la(L.kc) + pc_lb(L.kc);
-    if (ctx->eri_method == UNOMOL_ERI_MD || lsum > 8 || !fock_mixed_fused(L.bc, L.kc)) {
+    if (ctx->eri_method == UNOMOL_ERI_MD || lsum > 8 || !fock_split_class(L.bc, L.kc)) {
         ++launches;
         return launch_class_kernel(ctx, L, uhf, false, A, sl);
     }
@@ -694,7 +694,7 @@ cudaError_t launch_plain_class(const UnomolCtx* ctx, size_t li, bool uhf, FockAr
         A.dyn_count = ctx->d_cnt_lo + L.bp_begin;
         A.dyn_begin = ctx->d_begin_lo + L.bp_begin;
         A.dyn_total = ctx->d_total_lo + li;
-        e = launch_fock_df64(L.bc, L.kc, uhf, A, lo, ctx->nt, ctx->d_rysdf, sl);
+        e = launch_fock_df64(L.bc, L.kc, uhf, A, lo, ctx->nt, sl);
         ++launches;
     }
     return e;
@@ -739,6 +739,7 @@ int fock_device(UnomolCtx* ctx, const double* dPa, const double* dPb, double* dG
     A.prims = ctx->d_prims;
     A.prims32 = ctx->d_prims32;
     A.primsdf = ctx->d_primsdf;
+    A.rysdf = ctx->d_rysdf;
     A.nbf = n;
     A.Pa = ctx->d_Pa;
     A.Pb = uhf ? ctx->d_Pb : nullptr;
@@ -772,7 +773,7 @@ int fock_device(UnomolCtx* ctx, const double* dPa, const double* dPb, double* dG
         A.dmax = ctx->d_dmax;
         A.skip_cut = ctx->skip_cut;
         A.skip_cut32 = (float)ctx->skip_cut;
-        A.fp32_cut32 = ctx->fp32_cut > ctx->skip_cut ? (float)ctx->fp32_cut : 0.f;  // per-quartet FP32 choice (fused kernel)
+        A.fp32_cut32 = ctx->fp32_cut > ctx->skip_cut ? (float)ctx->fp32_cut : 0.f;  // per-quartet FP32 choice of the FP64 part
         A.dyn_mseg = ctx->d_mseg;
         CU(wl_to_float(ctx->d_Pa, ctx->d_Pa32, n2, s));
         A.Pa32 = ctx->d_Pa32;
@@ -792,18 +793,12 @@ int fock_device(UnomolCtx* ctx, const double* dPa, const double* dPb, double* dG
     }
     // one class: the reference's integral method (Rys for la+lb+lc+ld <= 8, MD above:
     // TwoElectronInts.cpp:658-666; MD everywhere in the MD mode), templated kernels for s/p/d
-#ifndef UGB_FUSED_MIXED
-#define UGB_FUSED_MIXED 1
-#endif
-#ifndef UGB_FUSE_MAXL
-#define UGB_FUSE_MAXL -1  // classes with la+lb+lc+ld above this run their two parts as separate kernels
-#endif                    // (-1: every class; the batched build keeps fused launches for (ss|ss), (ps|ss))
     // mixed builds: the FP64-part kernels on a high-priority stream, the FP32 kernels on a second one, so
     // that the FP64 CTAs take the SMs first and the FP32 CTAs fill the rest (213 vs 206 builds/s with the
     // classes alternating over two equal-priority streams); plain builds alternate their classes over two
     // streams
     const bool split = mixed && ctx->fp32_cut > ctx->skip_cut;
-    const bool fused = split && UGB_FUSED_MIXED && ctx->eri_method != UNOMOL_ERI_MD;
+    const bool templ = ctx->eri_method != UNOMOL_ERI_MD;
     cudaStream_t ls[2] = {s, s};  // streams of the FP64 and FP32 launches (plain builds: alternate classes)
     if (!ctx->counting) {
         CU(cudaEventRecord(ctx->fork, s));
@@ -831,7 +826,7 @@ int fock_device(UnomolCtx* ctx, const double* dPa, const double* dPb, double* dG
             A.dyn_begin = ctx->d_begin64 + L.bp_begin;
             A.dyn_total = ctx->d_total64 + li;
             const int lsum = pc_la(L.bc) + pc_lb(L.bc) + pc_la(L.kc) + pc_lb(L.kc);
-            if (fused && fock_mixed_fused(L.bc, L.kc) && lsum <= 8) {
+            if (templ && fock_split_class(L.bc, L.kc) && lsum <= 8) {
                 FockArgs A32 = A;
                 A32.mode = 2;
                 A32.dyn_prefix = ctx->d_pre32;
@@ -839,17 +834,14 @@ int fock_device(UnomolCtx* ctx, const double* dPa, const double* dPb, double* dG
                 A32.dyn_begin = ctx->d_begin32 + L.bp_begin;
                 A32.dyn_total = ctx->d_total32 + li;
                 A32.counter_base += ncls * 32;
-                if (lsum <= UGB_FUSE_MAXL) {
-                    CU(launch_fock_mixed(L.bc, L.kc, uhf, A, A32, ctx->nt, ctx->d_rys, ctx->d_rys32, ls[0]));
-                    ++launches;
-                } else {
-                    // classes whose FP32 code needs far fewer registers than their FP64 code: the FP64 part
-                    // (four lanes per quartet) and the FP32 part as two kernels on the two streams, each
-                    // at its own register count
-                    CU(launch_fock_fp64_part(L.bc, L.kc, uhf, A, A32, ctx->nt, ctx->d_rys, ctx->d_rys32, ctx->nsm * 4,
-                                             ls[0]));
+                // the FP64 part (four lanes per quartet), its quartets below SPLIT_CUT (pairs of floats) and the
+                // FP32 part as kernels of their own register counts
+                CU(launch_fock_fp64_part(L.bc, L.kc, uhf, A, A32, ctx->nt, ctx->d_rys, ctx->d_rys32, ctx->nsm * 4, ls[0]));
+                CU(launch_fock_df64_part(L.bc, L.kc, uhf, A, ctx->nt, ctx->nsm * 8, ls[0]));
+                launches += 2;
+                if (split) {
                     CU(launch_class_kernel(ctx, L, uhf, true, A32, ls[1]));
-                    launches += 2;
+                    ++launches;
                 }
                 continue;
             }
@@ -923,7 +915,7 @@ int fock_device(UnomolCtx* ctx, const double* dPa, const double* dPb, double* dG
                     n32 += q32[k];
                 }
                 // quartets the per-quartet density screen dropped do no quartet-level work; quartets of
-                // the FP64 part's lists that the fused kernel ran in FP32 count as FP32
+                // the FP64 part's lists run in FP32 count as FP32
                 long long d64 = 0, d32 = 0, dem = 0;
                 for (int k = 0; k < 32; ++k) {
                     d64 += (long long)c[(2 * ncls + cls) * 32 + k];
@@ -979,6 +971,7 @@ CtxView ctx_view(const UnomolCtx* c) {
     v.npairs = c->npairs;
     v.d_prims = c->d_prims;
     v.d_prims32 = c->d_prims32;
+    v.d_primsdf = c->d_primsdf;
     v.nprims = c->nprims;
     v.d_prefix = c->d_prefix;
     v.d_bps = c->d_bps;
@@ -994,6 +987,7 @@ CtxView ctx_view(const UnomolCtx* c) {
     v.nt = c->nt;
     v.d_rys = c->d_rys;
     v.d_rys32 = c->d_rys32;
+    v.d_rysdf = c->d_rysdf;
     return v;
 }
 
@@ -1473,6 +1467,7 @@ extern "C" int unomol_gpu_fock_rhf_noalloc(UnomolCtx* ctx, const double* dP, dou
     A.prims = ctx->d_prims;
     A.prims32 = ctx->d_prims32;
     A.primsdf = ctx->d_primsdf;
+    A.rysdf = ctx->d_rysdf;
     A.nbf = n;
     A.Pa = Pfull;
     A.Pb = nullptr;

@@ -23,6 +23,7 @@ struct CtxView {
     int npairs = 0;
     const PrimPair* d_prims = nullptr;
     const PrimPair32* d_prims32 = nullptr;
+    const PrimPairDF* d_primsdf = nullptr;
     long long nprims = 0;
     const long long* d_prefix = nullptr;
     const BlockPair* d_bps = nullptr;  // device block pairs (the class launches' ranges index them)
@@ -38,6 +39,7 @@ struct CtxView {
     NormTable nt{};
     const double* d_rys = nullptr;
     const float* d_rys32 = nullptr;
+    const float* d_rysdf = nullptr;
 };
 
 CtxView ctx_view(const UnomolCtx* ctx);

@@ -75,20 +75,21 @@ static_assert(SQRT_SRTERM * SQRT_SRTERM - SRTERM < 1e-13 && SRTERM - SQRT_SRTERM
 // descending Schwarz bound.
 struct ShellPair {
     int a_off, b_off;      // first AO of shell a (larger L) and of shell b
-    int la, lb;            // la >= lb
     int prim_begin, nprim; // primitive pair ik of this pair at prim_begin + ik * prim_stride
     int prim_stride;       // pairs of one block (equal nprim) interleave their primitive pairs: the
                            // stride is the block's pair count, so consecutive pairs' records are adjacent
-    int same;              // ish == jsh
+    signed char la, lb;    // la >= lb
+    signed char same;      // ish == jsh
     double AB[3];          // A - B
     double q;              // Schwarz bound: max over functions of sqrt|(ab|ab)|
     int ish, jsh;          // shell indices (ish >= jsh)
     int pad;
     float ABl[3];          // what A - B leaves over its FP32 copy, for the pairs-of-floats kernels
     float ABf[3];          // A - B and q in FP32, for the FP32 kernels (no FP64 work or conversion there)
-    float qf;
-    int spare_[2];         // 112 bytes
+    float qf;              // 96 bytes
 };
+
+static_assert(sizeof(ShellPair) == 96, "six 16-byte sectors a pair");
 
 // A rectangle (or triangle, when bra block == ket block) of quartets between two pair blocks,
 // trimmed by the Schwarz staircase: bra pair i pairs with the first cnt[i] ket pairs of its block.
@@ -108,6 +109,7 @@ struct FockArgs {
     const PrimPair* prims;
     const PrimPair32* prims32;
     const PrimPairDF* primsdf;
+    const float* rysdf;         // root tables of the pairs-of-floats kernels
     const BlockPair* bps;
     const long long* prefix;    // concatenated staircase prefix sums
     int nbp;                    // block pairs of this launch

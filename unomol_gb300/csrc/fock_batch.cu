@@ -8,19 +8,17 @@
 #include <climits>
 #include <cstring>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/unomol_gb300.h"
 #include "ctx_view.h"
+#include "fock_df64.cuh"
 #include "fock_dispatch.cuh"
 #include "setup.h"
 #include "worklists.h"
 
 using namespace ugb;
-
-#ifndef UGB_BATCH_FUSE_MAXL
-#define UGB_BATCH_FUSE_MAXL 1  // classes with la+lb+lc+ld above this launch their two parts separately
-#endif
 
 namespace {
 
@@ -28,7 +26,8 @@ template <int BC, int KC, typename R>
 cudaError_t persistent_one(const FockArgs& A, const NormTable& nt, const R* rys, int grid, int block, cudaStream_t s) {
     constexpr int LA = pc_la(BC), LB = pc_lb(BC), LC = pc_la(KC), LD = pc_lb(KC);
     if constexpr (QClass<LA, LB, LC, LD>::NF <= 81) {
-        fock_jk_persistent<LA, LB, LC, LD, false, R><<<grid, block, 0, s>>>(A, nt, rys);
+        if constexpr (sizeof(R) == 8) return cudaErrorInvalidValue;  // the split build's kernels
+        else fock_jk_persistent<LA, LB, LC, LD, false, R><<<grid, block, 0, s>>>(A, nt, rys);
     } else if constexpr (sizeof(R) == 8) {
         // large classes: one item per thread over the whole launch
         fock_jk_generic<false, double, PrimPair><<<(unsigned)((A.nwork + 63) / 64), 64, 0, s>>>(A, nt, rys, A.prims, LA, LB, LC, LD);
@@ -124,12 +123,20 @@ struct UnomolBatch {
     NormTable nt{};
     const double* rys = nullptr;
     const float* rys32 = nullptr;
+    const float* rysdf = nullptr;
     // precision form (UNOMOL_PREC_MIXED): per-build work lists as for one context, over all molecules
     int prec_mode = UNOMOL_PREC_FP64;
     double fp32_cut = 1e-10, skip_cut = 1e-13;
     long long nrows = 0, pmax_total = 0;
     int nbps = 0;
     PrimPair32* d_prims32 = nullptr;
+    PrimPairDF* d_primsdf = nullptr;
+    // the FP64 build's split at SPLIT_CUT over the merged staircases (as one context's): one allocation
+    char* d_split = nullptr;
+    long long *d_pre_hi = nullptr, *d_pre_lo = nullptr, *d_cnt_hi = nullptr, *d_cnt_lo = nullptr;
+    long long *d_begin_hi = nullptr, *d_begin_lo = nullptr, *d_total_hi = nullptr, *d_total_lo = nullptr;
+    int* d_mseg_hi = nullptr;
+    std::vector<long long> total_hi, total_lo;
     float* d_Pfull32 = nullptr;
     float *d_pmax = nullptr, *d_dmax = nullptr;
     int *d_nshell = nullptr, *d_shell0 = nullptr, *d_soff = nullptr, *d_sl = nullptr;
@@ -185,17 +192,46 @@ FockArgs batch_args(UnomolBatch* b, const BLaunch& L, int k) {
     A.tile_counter = b->d_tiles + 2 * k;
     A.mode = 0;
     A.prims32 = b->d_prims32;
+    A.primsdf = b->d_primsdf;
+    A.rysdf = b->rysdf;
     A.Pa32 = b->d_Pfull32;
     A.pmax = b->d_pmax;
     A.dmax = b->d_dmax;
     A.skip_cut = b->skip_cut;
     A.skip_cut32 = (float)b->skip_cut;
     A.fp32_cut = b->fp32_cut;
-    A.fp32_cut32 = b->fp32_cut > b->skip_cut ? (float)b->fp32_cut : 0.f;  // per-quartet FP32 choice of the fused kernel
+    A.fp32_cut32 = b->fp32_cut > b->skip_cut ? (float)b->fp32_cut : 0.f;  // per-quartet FP32 choice of the FP64 part
     A.dyn_mseg = b->d_mseg;
     A.mol_nshell = b->d_nshell;
     A.mol_pmax = b->d_pmax_off;
     return A;
+}
+
+// Arguments of one part of the FP64 build's split of launch k (above SPLIT_CUT: mode 3, below: mode 4).
+FockArgs split_args(UnomolBatch* b, const BLaunch& L, int k, bool above) {
+    FockArgs A = batch_args(b, L, k);
+    A.mode = above ? 3 : 4;
+    A.dyn_mseg = b->d_mseg_hi;
+    A.dyn_prefix = above ? b->d_pre_hi : b->d_pre_lo;
+    A.dyn_count = (above ? b->d_cnt_hi : b->d_cnt_lo) + L.bp_begin;
+    A.dyn_begin = (above ? b->d_begin_hi : b->d_begin_lo) + L.bp_begin;
+    A.dyn_total = (above ? b->d_total_hi : b->d_total_lo) + k;
+    return A;
+}
+
+// One class of the FP64 build: the quartets at or above SPLIT_CUT in FP64 on s0, the others in pairs of
+// floats (persistent tiles) on s1; the large d classes as one launch.
+cudaError_t batch_plain_class(UnomolBatch* b, const BLaunch& L, int k, cudaStream_t s0, cudaStream_t s1) {
+    if (!fock_split_class(L.bc, L.kc))
+        return launch_persistent(L.bc, L.kc, batch_args(b, L, k), b->nt, b->rys, b->nsm * L.ctas_per_sm, L.block, s0);
+    cudaError_t e = cudaSuccess;
+    const long long hi = b->total_hi[k], lo = b->total_lo[k];
+    if (hi > 0)
+        e = launch_fock_fp64_group(L.bc, L.kc, false, split_args(b, L, k, true), hi, true, hi <= (long long)b->nsm * 32 ? 32 : 4,
+                                   b->nt, b->rys, s0);
+    if (e == cudaSuccess && lo > 0)
+        e = launch_fock_df64_persistent(L.bc, L.kc, split_args(b, L, k, false), b->nt, b->nsm * L.ctas_per_sm, L.block, s1);
+    return e;
 }
 
 // the batched build on stream s (persistent launches); G = G(P) for every molecule
@@ -220,11 +256,11 @@ int batch_build(UnomolBatch* b, cudaStream_t s) {
                              b->d_total64, b->d_total32, s));
         BCU(wl_to_float(b->d_Pfull, b->d_Pfull32, b->dense_total, s));
     }
-    // the FP64 and the FP32 parts on two streams forked from s (joined before the fold): their persistent
-    // CTAs share the SMs, one kind on the FP64 pipe, the other on the FP32 pipe and the loads
+    // the FP64 and the FP32 (or pairs-of-floats) parts on two streams forked from s (joined before the fold):
+    // their CTAs share the SMs, one kind on the FP64 pipe, the other on the FP32 pipe and the loads
     const bool split = mixed && b->fp32_cut > b->skip_cut;
     cudaStream_t ls[2] = {s, s};
-    if (split) {
+    if (split || !mixed) {
         BCU(cudaEventRecord(b->fork, s));
         for (int q = 0; q < 2; ++q) {
             BCU(cudaStreamWaitEvent(b->part_stream[q], b->fork, 0));
@@ -235,7 +271,7 @@ int batch_build(UnomolBatch* b, cudaStream_t s) {
         const BLaunch& L = b->launches[k];
         FockArgs A = batch_args(b, L, (int)k);
         if (!mixed) {
-            BCU(launch_persistent(L.bc, L.kc, A, b->nt, b->rys, b->nsm * L.ctas_per_sm, L.block, s));
+            BCU(batch_plain_class(b, L, (int)k, ls[0], ls[1]));
             continue;
         }
         A.mode = 1;  // FP64 part
@@ -243,25 +279,21 @@ int batch_build(UnomolBatch* b, cudaStream_t s) {
         A.dyn_count = b->d_cnt64 + L.bp_begin;
         A.dyn_begin = b->d_begin64 + L.bp_begin;
         A.dyn_total = b->d_total64 + k;
-        // both parts of a templated class in one grid launch with alternating CTAs (fock_jk_mixed, as for
-        // one molecule; the merged work lists balance the molecules): 14 % faster than the two persistent
-        // parts for the 32-water cluster, the same for 256 molecules
-        if (split && fock_mixed_fused(L.bc, L.kc)) {
+        // as for one molecule: the FP64 part (four lanes per quartet), its quartets below SPLIT_CUT (pairs of
+        // floats) and the FP32 part (persistent) as kernels of their own, classes alternating over the streams
+        // (the light classes' two parts in one launch of alternating CTAs: 31.4 against 30.9 ms)
+        if (fock_split_class(L.bc, L.kc)) {
             FockArgs A32 = A;
             A32.mode = 2;
             A32.dyn_prefix = b->d_pre32;
             A32.dyn_count = b->d_cnt32 + L.bp_begin;
             A32.dyn_begin = b->d_begin32 + L.bp_begin;
             A32.dyn_total = b->d_total32 + k;
-            if (pc_la(L.bc) + pc_lb(L.bc) + pc_la(L.kc) + pc_lb(L.kc) <= UGB_BATCH_FUSE_MAXL) {
-                BCU(launch_fock_mixed(L.bc, L.kc, false, A, A32, b->nt, b->rys, b->rys32, ls[k & 1]));
-            } else {
-                // as for one molecule: the heavier classes' FP64 part (four lanes per quartet) and FP32 part
-                // (persistent) as two kernels on the two streams, each at its own register count
-                BCU(launch_fock_fp64_part(L.bc, L.kc, false, A, A32, b->nt, b->rys, b->rys32, b->nsm * 8, ls[k & 1]));
-                A32.tile_counter = b->d_tiles + 2 * k + 1;
+            BCU(launch_fock_fp64_part(L.bc, L.kc, false, A, A32, b->nt, b->rys, b->rys32, b->nsm * 8, ls[k & 1]));
+            BCU(launch_fock_df64_part(L.bc, L.kc, false, A, b->nt, b->nsm * 16, ls[k & 1]));
+            A32.tile_counter = b->d_tiles + 2 * k + 1;
+            if (split)
                 BCU(launch_persistent(L.bc, L.kc, A32, b->nt, b->rys32, b->nsm * L.ctas_per_sm, L.block, ls[(k + 1) & 1]));
-            }
             continue;
         }
         BCU(launch_persistent(L.bc, L.kc, A, b->nt, b->rys, b->nsm * L.ctas_per_sm, L.block, ls[0]));
@@ -275,7 +307,7 @@ int batch_build(UnomolBatch* b, cudaStream_t s) {
             BCU(launch_persistent(L.bc, L.kc, A, b->nt, b->rys32, b->nsm * L.ctas_per_sm, L.block, ls[1]));
         }
     }
-    if (split)
+    if (ls[0] != s)
         for (int q = 0; q < 2; ++q) {
             BCU(cudaEventRecord(b->join[q], ls[q]));
             BCU(cudaStreamWaitEvent(s, b->join[q], 0));
@@ -283,6 +315,58 @@ int batch_build(UnomolBatch* b, cudaStream_t s) {
     batch_fold<<<(unsigned)((b->packed_total + 255) / 256), 256, 0, s>>>(b->d_T, b->d_doff, b->d_G, b->d_poff, b->d_nbf,
                                                                          nmol, b->packed_total);
     BCU(cudaGetLastError());
+    return UNOMOL_OK;
+}
+
+// The split of the merged staircases at SPLIT_CUT (build_worklists does the same for one context).
+int make_split(UnomolBatch* b) {
+    const int nmol = (int)b->mols.size(), nl = (int)b->launches.size();
+    if (nl == 0) return UNOMOL_OK;
+    const size_t nr = (size_t)b->nrows, nbp = (size_t)b->nbps;
+    const size_t words = 2 * nr + 4 * nbp + 2 * (size_t)nl;
+    BCU(cudaMalloc(&b->d_split, words * sizeof(long long) + nr * sizeof(int)));
+    long long* p = reinterpret_cast<long long*>(b->d_split);
+    for (auto& q : {std::make_pair(&b->d_pre_hi, nr), {&b->d_pre_lo, nr}, {&b->d_cnt_hi, nbp}, {&b->d_cnt_lo, nbp},
+                    {&b->d_begin_hi, nbp}, {&b->d_begin_lo, nbp}, {&b->d_total_hi, (size_t)nl}, {&b->d_total_lo, (size_t)nl}}) {
+        *q.first = p;
+        p += q.second;
+    }
+    b->d_mseg_hi = reinterpret_cast<int*>(p);
+    // scratch of the two passes: row counts, row -> block pair, density bounds of one, launch ranges
+    std::vector<int> launch_bp;
+    for (const BLaunch& L : b->launches) {
+        launch_bp.push_back(L.bp_begin);
+        launch_bp.push_back(L.nbp);
+    }
+    const std::vector<float> one(nmol, 1.f);
+    char* tmp = nullptr;
+    BCU(cudaMalloc(&tmp, 2 * nr * sizeof(long long) + nr * sizeof(int) + nmol * sizeof(float) + launch_bp.size() * sizeof(int)));
+    long long* c64 = reinterpret_cast<long long*>(tmp);
+    long long* c32 = c64 + nr;
+    int* rowbp = reinterpret_cast<int*>(c32 + nr);
+    float* d_one = reinterpret_cast<float*>(rowbp + nr);
+    int* d_lbp = reinterpret_cast<int*>(d_one + nmol);
+    cudaStream_t s = b->stream;
+    std::vector<long long> tot(2 * (size_t)nl);
+    cudaError_t e = cudaSuccess;
+    auto ck = [&](cudaError_t x) {
+        if (e == cudaSuccess) e = x;
+    };
+    ck(cudaMemcpyAsync(d_one, one.data(), nmol * sizeof(float), cudaMemcpyHostToDevice, s));
+    ck(cudaMemcpyAsync(d_lbp, launch_bp.data(), launch_bp.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+    ck(cudaMemsetAsync(c64, 0, 2 * nr * sizeof(long long), s));
+    ck(cudaMemsetAsync(b->d_mseg_hi, 0, nr * sizeof(int), s));
+    ck(cudaMemsetAsync(rowbp, 0xff, nr * sizeof(int), s));
+    ck(setup_row_bp(b->d_bps, b->nbps, rowbp, s));
+    ck(wl_split_rows(b->d_pairs, b->d_bps, rowbp, b->d_prefix, b->nrows, d_one, SPLIT_CUT, 0.0, c64, c32, b->d_mseg_hi, s));
+    ck(wl_scan_rows(b->d_bps, b->nbps, c64, c32, b->d_pre_hi, b->d_pre_lo, b->d_cnt_hi, b->d_cnt_lo, s));
+    ck(wl_scan_launches(d_lbp, nl, b->d_cnt_hi, b->d_cnt_lo, b->d_begin_hi, b->d_begin_lo, b->d_total_hi, b->d_total_lo, s));
+    ck(cudaMemcpyAsync(tot.data(), b->d_total_hi, tot.size() * sizeof(long long), cudaMemcpyDeviceToHost, s));
+    ck(cudaStreamSynchronize(s));
+    cudaFree(tmp);
+    BCU(e);
+    b->total_hi.assign(tot.begin(), tot.begin() + nl);
+    b->total_lo.assign(tot.begin() + nl, tot.end());
     return UNOMOL_OK;
 }
 
@@ -409,6 +493,7 @@ int unomol_gpu_batch_create(const UnomolBasisDesc* bases, int nmol, UnomolBatch*
             b->nt = v.nt;
             b->rys = v.d_rys;
             b->rys32 = v.d_rys32;
+            b->rysdf = v.d_rysdf;
             b->rys_compat = v.rys_compat;
         }
         if (npair_tot + v.npairs >= INT_MAX || nprim_tot + v.nprims >= INT_MAX || nrow_tot + v.nrows >= INT_MAX) {
@@ -479,6 +564,7 @@ int unomol_gpu_batch_create(const UnomolBasisDesc* bases, int nmol, UnomolBatch*
     for (auto& e : b->join) BCU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     BCU(cudaMalloc(&b->d_pairs, sizeof(ShellPair) * std::max<long long>(1, npair_tot)));
     BCU(cudaMalloc(&b->d_prims, sizeof(PrimPair) * std::max<long long>(1, nprim_tot)));
+    BCU(cudaMalloc(&b->d_primsdf, sizeof(PrimPairDF) * std::max<long long>(1, nprim_tot)));
     BCU(cudaMalloc(&b->d_bps, sizeof(BlockPair) * std::max<size_t>(1, bps.size())));
     BCU(cudaMalloc(&b->d_prefix, sizeof(long long) * std::max<long long>(1, nrow_tot)));
     // the molecules' device set-ups side by side: pairs point into the merged primitive array and carry
@@ -491,6 +577,9 @@ int unomol_gpu_batch_create(const UnomolBasisDesc* bases, int nmol, UnomolBatch*
         }
         if (v.nprims > 0)
             BCU(cudaMemcpyAsync(b->d_prims + prim0s[m], v.d_prims, sizeof(PrimPair) * v.nprims, cudaMemcpyDeviceToDevice, b->stream));
+        if (v.nprims > 0)
+            BCU(cudaMemcpyAsync(b->d_primsdf + prim0s[m], v.d_primsdf, sizeof(PrimPairDF) * v.nprims, cudaMemcpyDeviceToDevice,
+                                b->stream));
         if (v.nrows > 0)
             BCU(cudaMemcpyAsync(b->d_prefix + row0s[m], v.d_prefix, sizeof(long long) * v.nrows, cudaMemcpyDeviceToDevice, b->stream));
     }
@@ -510,6 +599,10 @@ int unomol_gpu_batch_create(const UnomolBasisDesc* bases, int nmol, UnomolBatch*
     BCU(cudaMemcpy(b->d_doff, b->doff.data(), sizeof(long long) * nmol, cudaMemcpyHostToDevice));
     BCU(cudaMemcpy(b->d_poff, b->poff.data(), sizeof(long long) * nmol, cudaMemcpyHostToDevice));
     BCU(cudaMemset(b->d_P, 0, sizeof(double) * packed));
+    {
+        const int rc = make_split(b);
+        if (rc) return cleanup(rc);
+    }
     *out = b;
     return UNOMOL_OK;
 }
@@ -600,9 +693,11 @@ int unomol_gpu_batch_autotune(UnomolBatch* b, int reps, int* chosen) {
                 float tot = 0.f;
                 for (int r = 0; r < reps; ++r) {
                     BCU(cudaMemsetAsync(b->d_tiles + 2 * k, 0, sizeof(unsigned long long), s));
-                    FockArgs A = batch_args(b, L, (int)k);
                     BCU(cudaEventRecord(e0, s));
-                    BCU(launch_persistent(L.bc, L.kc, A, b->nt, b->rys, b->nsm * c, blk, s));
+                    if (fock_split_class(L.bc, L.kc))
+                        BCU(launch_fock_df64_persistent(L.bc, L.kc, split_args(b, L, (int)k, false), b->nt, b->nsm * c, blk, s));
+                    else
+                        BCU(launch_persistent(L.bc, L.kc, batch_args(b, L, (int)k), b->nt, b->rys, b->nsm * c, blk, s));
                     BCU(cudaEventRecord(e1, s));
                     BCU(cudaEventSynchronize(e1));
                     float ms = 0.f;
@@ -664,6 +759,8 @@ void unomol_gpu_batch_destroy(UnomolBatch* b) {
     dfree(b->d_Pfull);
     dfree(b->d_T);
     dfree(b->d_prims32);
+    dfree(b->d_primsdf);
+    dfree(b->d_split);
     dfree(b->d_Pfull32);
     dfree(b->d_pmax);
     dfree(b->d_dmax);

@@ -10,11 +10,22 @@
 namespace ugb {
 
 template <int BC, int KC, bool UHF>
-static cudaError_t launch_df(const FockArgs& A, long long items, const NormTable& nt, const float* tab, cudaStream_t s) {
+static cudaError_t launch_df(const FockArgs& A, long long items, const NormTable& nt, cudaStream_t s) {
     constexpr int LA = pc_la(BC), LB = pc_lb(BC), LC = pc_la(KC), LD = pc_lb(KC);
     if (items <= 0) return cudaSuccess;
     if constexpr (QClass<LA, LB, LC, LD>::NF <= 81) {
-        fock_jk_df64<LA, LB, LC, LD, UHF><<<(unsigned)((items + FOCK_THREADS - 1) / FOCK_THREADS), FOCK_THREADS, 0, s>>>(A, nt, tab);
+        fock_jk_df64<LA, LB, LC, LD, UHF><<<(unsigned)((items + FOCK_THREADS - 1) / FOCK_THREADS), FOCK_THREADS, 0, s>>>(A, nt);
+        return cudaGetLastError();
+    } else {
+        return cudaErrorInvalidValue;
+    }
+}
+
+template <int BC, int KC>
+static cudaError_t launch_persist(const FockArgs& A, const NormTable& nt, int grid, int block, cudaStream_t s) {
+    constexpr int LA = pc_la(BC), LB = pc_lb(BC), LC = pc_la(KC), LD = pc_lb(KC);
+    if constexpr (QClass<LA, LB, LC, LD>::NF <= 81) {
+        fock_jk_df64_persistent<LA, LB, LC, LD, false><<<grid, block, 0, s>>>(A, nt);
         return cudaGetLastError();
     } else {
         return cudaErrorInvalidValue;
@@ -43,11 +54,25 @@ static cudaError_t launch_group(const FockArgs& A, long long items, bool dyn, in
 
 #define UGB_CASE(BC, KC)                                                              \
     case (BC) * 8 + (KC):                                                             \
-        return uhf ? launch_df<BC, KC, true>(A, items, nt, tab, stream)              \
-                   : launch_df<BC, KC, false>(A, items, nt, tab, stream);
+        return uhf ? launch_df<BC, KC, true>(A, items, nt, stream)              \
+                   : launch_df<BC, KC, false>(A, items, nt, stream);
 
 cudaError_t launch_fock_df64(int bc, int kc, bool uhf, const FockArgs& A, long long items, const NormTable& nt,
-                             const float* tab, cudaStream_t stream) {
+                             cudaStream_t stream) {
+    switch (bc * 8 + kc) {
+#include "fock_cases.inc"
+        default:
+            return cudaErrorInvalidValue;
+    }
+}
+
+#undef UGB_CASE
+#define UGB_CASE(BC, KC)  \
+    case (BC) * 8 + (KC): \
+        return launch_persist<BC, KC>(A, nt, grid, block, stream);
+
+cudaError_t launch_fock_df64_persistent(int bc, int kc, const FockArgs& A, const NormTable& nt, int grid, int block,
+                                        cudaStream_t stream) {
     switch (bc * 8 + kc) {
 #include "fock_cases.inc"
         default:

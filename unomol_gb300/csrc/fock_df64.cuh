@@ -287,26 +287,51 @@ __device__ __forceinline__ void shell_quartet_df64(const ShellPair& bra, const S
     }
 }
 
-// The quartets below SPLIT_CUT of one class: integrals in double-float, density contraction and scatter in
-// FP64 as the FP64 kernels.
+// One quartet: integrals in pairs of floats, density contraction and scatter in FP64 as the FP64 kernels.
 template <int LA, int LB, int LC, int LD, bool UHF>
-__global__ void __launch_bounds__(128, LA + LB + LC + LD <= 1 ? 8 : 1) fock_jk_df64(const FockArgs A, const NormTable nt, const float* __restrict__ tab) {
+__device__ __forceinline__ void df_item(const FockArgs& A, const NormTable& nt, long long g) {
     using Q = QClass<LA, LB, LC, LD>;
     int bi, ki;
-    if (!decode_work_warp<true>(A, (long long)blockIdx.x * blockDim.x + threadIdx.x, bi, ki)) return;
+    if (!decode_work_warp<true>(A, g, bi, ki)) return;
     const ShellPair bra = A.pairs[bi];
     const ShellPair ket = A.pairs[ki];
+    if (A.mode == 1) {  // the FP64 part of a mixed build: the others are the group kernel's
+        if (!(bra.qf * ket.qf < float(SPLIT_CUT))) return;
+        const float bound = quartet_bound(A, bra, ket);
+        if (bound < A.skip_cut32 || bound < A.fp32_cut32) return;
+    }
     unsigned npass = 0;
     double v[Q::NF];
     {
         df acc[Q::NF];
-        shell_quartet_df64<LA, LB, LC, LD>(bra, ket, A.primsdf, tab, A.prim_cut32, A.rys_compat != 0, acc,
+        shell_quartet_df64<LA, LB, LC, LD>(bra, ket, A.primsdf, A.rysdf, A.prim_cut32, A.rys_compat != 0, acc,
                                            A.counters ? &npass : nullptr);
 #pragma unroll
         for (int f = 0; f < Q::NF; ++f) v[f] = df_to_f64(acc[f]);
     }
     digest_jk<LA, LB, LC, LD, UHF, double>(A, bra, ket, bi == ki, v, nt);
     if (A.counters) count_flush(A, npass);
+}
+
+// The quartets below SPLIT_CUT of one class (its split list).
+template <int LA, int LB, int LC, int LD, bool UHF>
+__global__ void __launch_bounds__(128, LA + LB + LC + LD <= 1 ? 8 : 1) fock_jk_df64(const FockArgs A, const NormTable nt) {
+    df_item<LA, LB, LC, LD, UHF>(A, nt, (long long)blockIdx.x * blockDim.x + threadIdx.x);
+}
+
+// The same for batches of molecules: a fixed grid pulling tiles (fock_jk_persistent).
+template <int LA, int LB, int LC, int LD, bool UHF>
+__global__ void __launch_bounds__(256, LA + LB + LC + LD <= 1 ? 4 : 1) fock_jk_df64_persistent(const FockArgs A, const NormTable nt) {
+    __shared__ long long tile;
+    const long long end = *A.dyn_total;
+    for (;;) {
+        if (threadIdx.x == 0) tile = (long long)atomicAdd(A.tile_counter, 1ull);
+        __syncthreads();
+        const long long g0 = tile * blockDim.x;
+        __syncthreads();
+        if (g0 >= end) return;
+        df_item<LA, LB, LC, LD, UHF>(A, nt, g0 + threadIdx.x);
+    }
 }
 
 // FP64 integrals with NP lanes per shell quartet, each summing every NP-th primitive quartet: where a launch

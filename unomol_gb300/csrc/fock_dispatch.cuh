@@ -14,30 +14,34 @@ __host__ __device__ constexpr int pc_la(int c) { return (c >= 1) + (c >= 3) + (c
 __host__ __device__ constexpr int pc_lb(int c) { return c - pc_la(c) * (pc_la(c) + 1) / 2; }
 
 // Launches the Fock kernel of quartet class (bc | kc) over `A.nwork` work items on `stream`.
-// Returns cudaSuccess or the launch error.
+// Returns cudaSuccess or the launch error.  FP64: the classes that fock_split_class does not accept.
 cudaError_t launch_fock_fp64(int bc, int kc, bool uhf, const FockArgs& A, const NormTable& nt,
                              const double* rys, cudaStream_t stream);
 cudaError_t launch_fock_fp32(int bc, int kc, bool uhf, const FockArgs& A, const NormTable& nt,
                              const float* rys, cudaStream_t stream);
-// Both parts of a mixed build of one class in one launch (their CTAs alternate); only for the classes
-// that fock_mixed_fused accepts (templated, at most 81 function quartets).
-bool fock_mixed_fused(int bc, int kc);
-cudaError_t launch_fock_mixed(int bc, int kc, bool uhf, const FockArgs& A64, const FockArgs& A32, const NormTable& nt,
-                              const double* rys64, const float* rys32, cudaStream_t stream);
-// The FP64 part of a mixed build of one class alone (classes that fock_mixed_fused accepts), on a grid of
+// Whether a class has the templated kernels of the split builds (s, p and d shells, at most 81 function
+// quartets).
+bool fock_split_class(int bc, int kc);
+// The FP64 part of a mixed build of one class alone (fock_split_class), on a grid of
 // at most `grid` CTAs whose warps step over the part's quartets (NP lanes per quartet).
 cudaError_t launch_fock_fp64_part(int bc, int kc, bool uhf, const FockArgs& A64, const FockArgs& A32, const NormTable& nt,
                                   const double* rys64, const float* rys32, int grid, cudaStream_t stream);
+// That part's quartets in pairs of floats as a kernel of their own.
+cudaError_t launch_fock_df64_part(int bc, int kc, bool uhf, const FockArgs& A, const NormTable& nt, int grid,
+                                  cudaStream_t stream);
 cudaError_t launch_schwarz(int pc, const ShellPair* pairs, const PrimPair* prims, int begin, int count,
                            const NormTable& nt, const double* rys, double* q_out, cudaStream_t stream);
 
 // The quartets below SPLIT_CUT of one class in pairs of floats (fock_df64.cuh), `items` of its split list.
 cudaError_t launch_fock_df64(int bc, int kc, bool uhf, const FockArgs& A, long long items, const NormTable& nt,
-                             const float* tab, cudaStream_t stream);
+                             cudaStream_t stream);
+// The same over a fixed grid pulling tiles of `block` quartets (RHF; batches of molecules).
+cudaError_t launch_fock_df64_persistent(int bc, int kc, const FockArgs& A, const NormTable& nt, int grid, int block,
+                                        cudaStream_t stream);
 // One class in FP64 with `lanes` (4 or 32) lanes per quartet: `items` of a split list (dyn) or of the whole class.
 cudaError_t launch_fock_fp64_group(int bc, int kc, bool uhf, const FockArgs& A, long long items, bool dyn, int lanes,
                                    const NormTable& nt, const double* rys, cudaStream_t stream);
-// Both take the classes that fock_mixed_fused accepts.  The root tables of the first:
+// All for the classes that fock_split_class accepts.  The root tables of the first:
 std::vector<float> df_rys_tables();
 
 // Runtime-L Rys kernel (classes with f or g shells and la+lb+lc+ld <= 8), FP64 or FP32.

@@ -1,4 +1,4 @@
-// FP64 instances of the class-templated Fock kernels (the plain path) and the Schwarz diagonal.
+// FP64 launches of the large d classes (runtime loops) and the Schwarz diagonal.
 #include "fock_kernels.cuh"
 #include "fock_dispatch.cuh"
 
@@ -9,13 +9,12 @@ static cudaError_t launch_one(const FockArgs& A, const NormTable& nt, const doub
     constexpr int LA = pc_la(BC), LB = pc_lb(BC), LC = pc_la(KC), LD = pc_lb(KC);
     if (A.nwork <= 0) return cudaSuccess;
     if constexpr (QClass<LA, LB, LC, LD>::NF <= 81) {
-        const long long blocks = (A.nwork + FOCK_THREADS - 1) / FOCK_THREADS;
-        fock_jk_kernel<LA, LB, LC, LD, UHF, double><<<(unsigned)blocks, FOCK_THREADS, 0, s>>>(A, nt, rys);
+        return cudaErrorInvalidValue;  // the split build's kernels (fock_df64.cu, fock_mixed.cu)
     } else {
         const long long blocks = (A.nwork + 63) / 64;
         fock_jk_generic<UHF, double, PrimPair><<<(unsigned)blocks, 64, 0, s>>>(A, nt, rys, A.prims, LA, LB, LC, LD);
+        return cudaGetLastError();
     }
-    return cudaGetLastError();
 }
 
 #define UGB_CASE(BC, KC)                                                              \

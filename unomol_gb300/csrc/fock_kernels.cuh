@@ -780,32 +780,6 @@ __device__ __forceinline__ void fock_item(const FockArgs& A, const NormTable& nt
     quartet_item<LA, LB, LC, LD, UHF, R>(A, nt, rys, bra, ket, bi == ki);
 }
 
-// FP64 part of a mixed build, with the precision chosen per quartet.  The work lists put a quartet in
-// the FP64 part when its Schwarz bound times the largest |P| of the whole density reaches the FP32 cut;
-// here a quartet whose bound times the largest |P| of its own six blocks (the density elements it is
-// contracted with) is below that cut runs in FP32 (with the FP32 part's arguments A32), under the same
-// per-quartet error bound as the FP32 part's own quartets.
-template <int LA, int LB, int LC, int LD, bool UHF>
-__device__ __forceinline__ void fock_item_fp64_part(const FockArgs& A64, const FockArgs& A32, const NormTable& nt,
-                                                    const double* __restrict__ rys64, const float* __restrict__ rys32,
-                                                    long long g) {
-    int bi, ki;
-    if (!decode_work_warp<true>(A64, g, bi, ki)) return;
-    const ShellPair bra = A64.pairs[bi];
-    const ShellPair ket = A64.pairs[ki];
-    const float bound = quartet_bound(A64, bra, ket);
-    if (bound < A64.skip_cut32) {
-        if (A64.counters) count_screened(A64);
-        return;
-    }
-    if (bound < A64.fp32_cut32) {
-        if (A64.counters) count_demoted(A64);
-        quartet_item<LA, LB, LC, LD, UHF, float>(A32, nt, rys32, bra, ket, bi == ki);
-    } else {
-        quartet_item<LA, LB, LC, LD, UHF, double>(A64, nt, rys64, bra, ket, bi == ki);
-    }
-}
-
 // One shell quartet on a group of NP lanes (mask gmask): lane `part` of the group sums the primitive
 // quartets part, part + NP, ...; the group adds its partial integrals with warp shuffles and its first
 // lane contracts them with the density.
@@ -830,87 +804,9 @@ __device__ __forceinline__ void quartet_item_group(const FockArgs& A, const Norm
     if (A.counters) count_flush(A, npass);
 }
 
-// FP64 part of a mixed build with NP lanes per quartet: the warp holds the 32 / NP items from g0 (the FP64
-// part's quartets are few and the costliest of the build, so one lane per quartet leaves most of the
-// FP64 pipe's issue slots idle); precision chosen per quartet as in fock_item_fp64_part.
-template <int LA, int LB, int LC, int LD, bool UHF, int NP>
-__device__ __forceinline__ void fock_group_fp64_part(const FockArgs& A64, const FockArgs& A32, const NormTable& nt,
-                                                     const double* __restrict__ rys64, const float* __restrict__ rys32,
-                                                     long long g0) {
-    const int lane = threadIdx.x & 31, sub = lane / NP, part = lane % NP;
-    const unsigned gmask = ((1u << NP) - 1u) << (sub * NP);
-    int bi, ki;
-    if (!decode_warp_items<true>(A64, g0, sub, bi, ki)) return;  // warp-collective; uniform over a group
-    const ShellPair bra = A64.pairs[bi];
-    const ShellPair ket = A64.pairs[ki];
-    const float bound = quartet_bound(A64, bra, ket);
-    if (bound < A64.skip_cut32) {
-        if (A64.counters && part == 0) count_screened(A64);
-        return;
-    }
-    if (bound < A64.fp32_cut32) {
-        if (A64.counters && part == 0) count_demoted(A64);
-        quartet_item_group<LA, LB, LC, LD, UHF, float, NP>(A32, nt, rys32, bra, ket, bi == ki, part, gmask);
-    } else {
-        quartet_item_group<LA, LB, LC, LD, UHF, double, NP>(A64, nt, rys64, bra, ket, bi == ki, part, gmask);
-    }
-}
-
-#ifndef UGB_FP64_PARTS
-#define UGB_FP64_PARTS 4
-#endif
-// Lanes per quartet of the FP64 part of a mixed build
-template <int LA, int LB, int LC, int LD>
-struct Fp64Parts {
-    static constexpr int value = UGB_FP64_PARTS;
-};
-
 template <int LA, int LB, int LC, int LD, bool UHF, typename R>
 __global__ void __launch_bounds__(128) fock_jk_kernel(const FockArgs A, const NormTable nt, const R* __restrict__ rys) {
     fock_item<LA, LB, LC, LD, UHF, R>(A, nt, rys, (long long)blockIdx.x * blockDim.x + threadIdx.x);
-}
-
-// Mixed builds: the FP64 part (A64, mode 1) and the FP32 part (A32, mode 2) of one class in one launch
-// of 2 x nblk CTAs, alternating (even CTAs FP64, odd CTAs FP32).  Both parts number their quartets
-// compactly from 0, so their working CTAs come first in the grid and an SM holds both kinds at once:
-// warps on the FP64 pipe beside warps on the FP32 pipe and the loads.  CTAs past a part's total end at
-// their first load.  The FP64 part's quartets whose own density bound is below the FP32 cut run in FP32
-// (fock_item_fp64_part).
-template <int LA, int LB, int LC, int LD, bool UHF>
-__global__ void __launch_bounds__(128) fock_jk_mixed(const FockArgs A64, const FockArgs A32, const NormTable nt,
-                                                      const double* __restrict__ rys64,
-                                                      const float* __restrict__ rys32) {
-    const long long g = (long long)(blockIdx.x >> 1) * blockDim.x + threadIdx.x;
-    if (blockIdx.x & 1) {
-        fock_item<LA, LB, LC, LD, UHF, float>(A32, nt, rys32, g);
-        return;
-    }
-    constexpr int NP = Fp64Parts<LA, LB, LC, LD>::value;
-    if constexpr (NP == 1) {
-        fock_item_fp64_part<LA, LB, LC, LD, UHF>(A64, A32, nt, rys64, rys32, g);
-    } else {
-        // the FP64 CTAs cover 32 / NP items per warp and step over the part's total in whole warps
-        const long long per_warp = 32 / NP;
-        const long long nwarps = (long long)((gridDim.x + 1) >> 1) * (blockDim.x >> 5);
-        const long long total = *A64.dyn_total;
-        for (long long wi = (long long)(blockIdx.x >> 1) * (blockDim.x >> 5) + (threadIdx.x >> 5); wi * per_warp < total;
-             wi += nwarps)
-            fock_group_fp64_part<LA, LB, LC, LD, UHF, NP>(A64, A32, nt, rys64, rys32, wi * per_warp);
-    }
-}
-
-// The FP64 part of a mixed build alone (NP lanes per quartet, per-quartet precision as in fock_jk_mixed),
-// for the classes whose FP32 part runs as its own kernel at the FP32 code's register count: a fixed grid
-// whose warps step over the part's quartets.
-template <int LA, int LB, int LC, int LD, bool UHF>
-__global__ void __launch_bounds__(128) fock_jk_fp64_part(const FockArgs A64, const FockArgs A32, const NormTable nt,
-                                                         const double* __restrict__ rys64, const float* __restrict__ rys32) {
-    constexpr int NP = Fp64Parts<LA, LB, LC, LD>::value;
-    const long long per_warp = 32 / NP;
-    const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
-    const long long total = *A64.dyn_total;
-    for (long long wi = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); wi * per_warp < total; wi += nwarps)
-        fock_group_fp64_part<LA, LB, LC, LD, UHF, NP>(A64, A32, nt, rys64, rys32, wi * per_warp);
 }
 
 // Persistent form for batches of molecules: a fixed grid of CTAs (a few per SM) pulls tiles of
