@@ -109,8 +109,8 @@ struct UnomolCtx {
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     // mixed builds: the FP64 and the FP32 parts on two side streams forked from and joined back into
     // the build's stream, so that the two kinds of kernels (FP64 pipe / FP32 pipe and loads) share the SMs
-    cudaStream_t part_stream[3] = {nullptr, nullptr, nullptr};  // FP64 part, FP32 part, second plain stream
-    cudaEvent_t fork = nullptr, join[2] = {nullptr, nullptr};
+    cudaStream_t part_stream[3] = {nullptr, nullptr, nullptr};  // FP64 part; FP32 or pairs-of-floats part, two streams
+    cudaEvent_t fork = nullptr, join[3] = {nullptr, nullptr, nullptr};
     // options
     double schwarz_cut = STORE_CUT;
     int prec_mode = UNOMOL_PREC_FP64;
@@ -793,18 +793,18 @@ int fock_device(UnomolCtx* ctx, const double* dPa, const double* dPb, double* dG
     }
     // one class: the reference's integral method (Rys for la+lb+lc+ld <= 8, MD above:
     // TwoElectronInts.cpp:658-666; MD everywhere in the MD mode), templated kernels for s/p/d
-    // mixed builds: the FP64-part kernels on a high-priority stream, the FP32 kernels on a second one, so
-    // that the FP64 CTAs take the SMs first and the FP32 CTAs fill the rest (213 vs 206 builds/s with the
-    // classes alternating over two equal-priority streams); plain builds alternate their classes over two
-    // streams
+    // the FP64 kernels on a high-priority stream, so that their CTAs take the SMs first, and the classes' FP32
+    // (or pairs-of-floats) kernels alternating over two low-priority ones, so that one class's last CTAs
+    // overlap the next class's first (n-decane UHF 3.54 -> 3.33 ms; 32 waters mixed, full density, 7.65 -> 7.57)
     const bool split = mixed && ctx->fp32_cut > ctx->skip_cut;
     const bool templ = ctx->eri_method != UNOMOL_ERI_MD;
-    cudaStream_t ls[2] = {s, s};  // streams of the FP64 and FP32 launches (plain builds: alternate classes)
+    cudaStream_t ls[3] = {s, s, s};
     if (!ctx->counting) {
         CU(cudaEventRecord(ctx->fork, s));
-        ls[0] = ctx->part_stream[0];
-        ls[1] = ctx->part_stream[1];
-        for (int k = 0; k < 2; ++k) CU(cudaStreamWaitEvent(ls[k], ctx->fork, 0));
+        for (int k = 0; k < 3; ++k) {
+            ls[k] = ctx->part_stream[k];
+            CU(cudaStreamWaitEvent(ls[k], ctx->fork, 0));
+        }
     }
     auto launch_class = [&](const ClassLaunch& L, bool fp32) -> cudaError_t {
         return launch_class_kernel(ctx, L, uhf, fp32, A, ls[fp32 ? 1 : 0]);
@@ -818,7 +818,7 @@ int fock_device(UnomolCtx* ctx, const double* dPa, const double* dPb, double* dG
         A.nwork = L.nwork;
         A.counter_base = (L.bc * NPAIRCLASS + L.kc) * 32;  // FP32 launches use the second half
         if (!mixed) {
-            CU(launch_plain_class(ctx, li, uhf, A, ls[0], ls[(lk & 1) ? 1 : 0], launches));
+            CU(launch_plain_class(ctx, li, uhf, A, ls[0], ls[1 + (lk & 1)], launches));
         } else {
             A.mode = 1;
             A.dyn_prefix = ctx->d_pre64;
@@ -840,7 +840,7 @@ int fock_device(UnomolCtx* ctx, const double* dPa, const double* dPb, double* dG
                 CU(launch_fock_df64_part(L.bc, L.kc, uhf, A, ctx->nt, ctx->nsm * 8, ls[0]));
                 launches += 2;
                 if (split) {
-                    CU(launch_class_kernel(ctx, L, uhf, true, A32, ls[1]));
+                    CU(launch_class_kernel(ctx, L, uhf, true, A32, ls[1 + (lk & 1)]));
                     ++launches;
                 }
                 continue;
@@ -860,7 +860,7 @@ int fock_device(UnomolCtx* ctx, const double* dPa, const double* dPb, double* dG
         }
     }
     if (ls[0] != s) {  // join the two parts back into the build's stream
-        for (int k = 0; k < 2; ++k) {
+        for (int k = 0; k < 3; ++k) {
             CU(cudaEventRecord(ctx->join[k], ls[k]));
             CU(cudaStreamWaitEvent(s, ctx->join[k], 0));
         }
@@ -1382,7 +1382,7 @@ void unomol_gpu_destroy(UnomolCtx* ctx) {
     dfree(ctx->d_Pb32);
     for (auto& e : ctx->ev)
         if (e) cudaEventDestroy(e);
-    for (cudaEvent_t e : {ctx->fork, ctx->join[0], ctx->join[1]})
+    for (cudaEvent_t e : {ctx->fork, ctx->join[0], ctx->join[1], ctx->join[2]})
         if (e) cudaEventDestroy(e);
     for (cudaStream_t st : ctx->part_stream)
         if (st) {

@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(128) gdpm_kernel(const ShellPair* __restrict__
 #pragma unroll
         for (int ib = 0; ib < Q::NB; ++ib) {
             const int i = bra.a_off + ia, j = bra.b_off + ib;
-            if (bra.same && j > i) continue;
+            if (bra.same() && j > i) continue;
             const int hi = i > j ? i : j, lo = i > j ? j : i;
             out[(long long)hi * (hi + 1) / 2 + lo] = acc[ia * Q::NB + ib] * nt.v[LA][ia] * nt.v[LB][ib];
         }

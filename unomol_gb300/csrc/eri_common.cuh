@@ -73,23 +73,28 @@ static_assert(SQRT_SRTERM * SQRT_SRTERM - SRTERM < 1e-13 && SRTERM - SQRT_SRTERM
 
 // One shell pair, sorted into blocks of equal (class, primitive-pair count), within a block by
 // descending Schwarz bound.
-struct ShellPair {
+struct __align__(8) ShellPair {
+    // the first and the third 32-byte sector are what the FP32 kernels read, in 8-byte loads (the fields one
+    // by one cost those kernels 2 %)
     int a_off, b_off;      // first AO of shell a (larger L) and of shell b
     int prim_begin, nprim; // primitive pair ik of this pair at prim_begin + ik * prim_stride
     int prim_stride;       // pairs of one block (equal nprim) interleave their primitive pairs: the
                            // stride is the block's pair count, so consecutive pairs' records are adjacent
-    signed char la, lb;    // la >= lb
-    signed char same;      // ish == jsh
+    int flags;             // bit 0: ish == jsh; la << 8, lb << 16 (la >= lb)
+    int pad;               // the molecule of a batch
+    float ABl0;            // ABl0..2: what A - B leaves over its FP32 copy, for the pairs-of-floats kernels
     double AB[3];          // A - B
     double q;              // Schwarz bound: max over functions of sqrt|(ab|ab)|
     int ish, jsh;          // shell indices (ish >= jsh)
-    int pad;
-    float ABl[3];          // what A - B leaves over its FP32 copy, for the pairs-of-floats kernels
+    float ABl1, ABl2;
     float ABf[3];          // A - B and q in FP32, for the FP32 kernels (no FP64 work or conversion there)
-    float qf;              // 96 bytes
+    float qf;
+    __host__ __device__ bool same() const { return flags & 1; }
+    __host__ __device__ int la() const { return (flags >> 8) & 0xff; }
+    __host__ __device__ int lb() const { return (flags >> 16) & 0xff; }
 };
 
-static_assert(sizeof(ShellPair) == 96, "six 16-byte sectors a pair");
+static_assert(sizeof(ShellPair) == 96, "three 32-byte sectors a pair");
 
 // A rectangle (or triangle, when bra block == ket block) of quartets between two pair blocks,
 // trimmed by the Schwarz staircase: bra pair i pairs with the first cnt[i] ket pairs of its block.

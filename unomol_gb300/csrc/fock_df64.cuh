@@ -162,6 +162,10 @@ __device__ __forceinline__ double df_to_f64(df a) {
     return cvt(a.h) + cvt(a.l);
 }
 
+__device__ __forceinline__ df pair_ab(const ShellPair& p, int k) {
+    return {p.ABf[k], k == 0 ? p.ABl0 : k == 1 ? p.ABl1 : p.ABl2};
+}
+
 // Contracted integrals of one shell quartet as shell_quartet_eri<..., double>, in double-float: the same
 // primitive quartets (prefactor screen on floats, decided in double-float within 0.1 % of the cut).
 template <int LA, int LB, int LC, int LD>
@@ -216,7 +220,7 @@ __device__ __forceinline__ void shell_quartet_df64(const ShellPair& bra, const S
                 const df nqf = df_neg(qf);
                 auto axis = [&](int k, const df& PQ, auto unit, df g, df(&I)[Q::NI]) {
                     const df C = L12 > 0 ? df_fma(nqf, PQ, bp.PA[k]) : zero, Cp = L34 > 0 ? df_fma(pf, PQ, kp.PA[k]) : zero;
-                    const df AB = LB > 0 ? df{bra.ABf[k], bra.ABl[k]} : zero, CD = LD > 0 ? df{ket.ABf[k], ket.ABl[k]} : zero;
+                    const df AB = LB > 0 ? pair_ab(bra, k) : zero, CD = LD > 0 ? pair_ab(ket, k) : zero;
                     df_axis<LA, LB, LC, LD, decltype(unit)::value>(g, C, Cp, B00, B1, B1p, AB, CD, I);
                 };
                 axis(0, PQx, std::true_type{}, df{1.f, 0.f}, Ix);

@@ -612,7 +612,7 @@ __device__ __forceinline__ void digest_jk(const FockArgs& A, const ShellPair& br
     double* __restrict__ Tb = UHF ? A.Tb + base : nullptr;
     // The degeneracy factor 1/2 per coincidence and the 4 (2) of the Coulomb sums are powers of two: applied
     // to the exponent fields, on the integer pipe (per (ss|ss) quartet 18 -> 7 FP64 instructions).
-    const int ndeg = (bra.same != 0) + (ket.same != 0) + (same_pair ? 1 : 0);
+    const int ndeg = (bra.same() ? 1 : 0) + (ket.same() ? 1 : 0) + (same_pair ? 1 : 0);
     const R* __restrict__ Pa;
     const R* __restrict__ Pb;
     if constexpr (sizeof(R) == 8) {
@@ -990,8 +990,8 @@ __global__ void __launch_bounds__(64) fock_jk_generic(const FockArgs A, const No
     double* __restrict__ Ta = A.Ta + base;
     double* __restrict__ Tb = UHF ? A.Tb + base : nullptr;
     double deg = 1.0;
-    if (bra.same) deg *= 0.5;
-    if (ket.same) deg *= 0.5;
+    if (bra.same()) deg *= 0.5;
+    if (ket.same()) deg *= 0.5;
     if (bi == ki) deg *= 0.5;
     const double* __restrict__ Pa = A.Pa + base;
     const double* __restrict__ Pb = UHF ? A.Pb + base : nullptr;
@@ -1047,7 +1047,7 @@ static __global__ void __launch_bounds__(64) schwarz_generic(const ShellPair* __
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= count) return;
     const ShellPair sp = pairs[begin + t];
-    const int la = sp.la, lb = sp.lb;
+    const int la = sp.la(), lb = sp.lb();
     const int NA = ncart(la), NB = ncart(lb);
     const int nr = (2 * la + 2 * lb) / 2 + 1;
     double acc[GEN_NC * GEN_NC];  // only the diagonal (ab|ab) is needed

@@ -91,7 +91,7 @@ static __global__ void __launch_bounds__(64) store_records_generic(const FockArg
                         const double v = acc[f] * (nt.v[la][ia] * nt.v[lb][ib] * nt.v[lc][ic] * nt.v[ld][id]);
                         if (!above_cut(v, A.thr_int)) continue;  // TwoElectronInts.cpp:668
                         int i, j, k, l;
-                        if (!canonical_label(bra.a_off + ia, bra.b_off + ib, ket.a_off + ic, ket.b_off + id, bra.same, ket.same,
+                        if (!canonical_label(bra.a_off + ia, bra.b_off + ib, ket.a_off + ic, ket.b_off + id, bra.same(), ket.same(),
                                              bi == ki, i, j, k, l))
                             continue;
                         if (pass == 0) ++n;
@@ -118,7 +118,7 @@ static __global__ void __launch_bounds__(128) store_records_md(const FockArgs A,
             const ShellPair bra = A.pairs[bi];
             const ShellPair ket = A.pairs[ki];
             const int id = f % ND, ic = (f / ND) % NC, ib = (f / (ND * NC)) % NB, ia = f / (ND * NC * NB);
-            if (canonical_label(bra.a_off + ia, bra.b_off + ib, ket.a_off + ic, ket.b_off + id, bra.same, ket.same, bi == ki, i,
+            if (canonical_label(bra.a_off + ia, bra.b_off + ib, ket.a_off + ic, ket.b_off + id, bra.same(), ket.same(), bi == ki, i,
                                 j, k, l)) {
                 v = md_function_quartet(bra, ket, A.prims, la, lb, lc, ld, ia, ib, ic, id);
                 v *= nt.v[la][ia] * nt.v[lb][ib] * nt.v[lc][ic] * nt.v[ld][id];

@@ -161,8 +161,8 @@ __global__ void __launch_bounds__(128) fock_jk_md(const FockArgs A, const NormTa
         v *= nt.v[la][ia] * nt.v[lb][ib] * nt.v[lc][ic] * nt.v[ld][id];
         if (!above_cut(v, A.thr_int)) continue;  // TwoElectronInts.cpp:668
         double deg = 1.0;
-        if (bra.same) deg *= 0.5;
-        if (ket.same) deg *= 0.5;
+        if (bra.same()) deg *= 0.5;
+        if (ket.same()) deg *= 0.5;
         if (bi == ki) deg *= 0.5;
         v *= deg;
         const int N = A.nbf;
@@ -198,13 +198,13 @@ __global__ void __launch_bounds__(128) schwarz_md(const ShellPair* __restrict__ 
                                                   int begin, int count, const NormTable nt, unsigned long long* qbits) {
     const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const ShellPair& s0 = pairs[begin];
-    const int nab = ncart(s0.la) * ncart(s0.lb);
+    const int nab = ncart(s0.la()) * ncart(s0.lb());
     if (g >= (long long)count * nab) return;
     const int t = (int)(g / nab), f = (int)(g % nab);
     const ShellPair sp = pairs[begin + t];
-    const int ia = f / ncart(sp.lb), ib = f % ncart(sp.lb);
-    double v = md_function_quartet(sp, sp, prims, sp.la, sp.lb, sp.la, sp.lb, ia, ib, ia, ib);
-    const double n = nt.v[sp.la][ia] * nt.v[sp.lb][ib];
+    const int ia = f / ncart(sp.lb()), ib = f % ncart(sp.lb());
+    double v = md_function_quartet(sp, sp, prims, sp.la(), sp.lb(), sp.la(), sp.lb(), ia, ib, ia, ib);
+    const double n = nt.v[sp.la()][ia] * nt.v[sp.lb()][ib];
     v = fabs(v) * n * n;
     atomicMax(qbits + begin + t, (unsigned long long)__double_as_longlong(v));
 }

@@ -53,9 +53,7 @@ __global__ void k_build_pairs(const ShellsDev sh, int npairs, const int* __restr
     sp.ish = ish;
     sp.jsh = jsh;
     sp.prim_stride = 1;  // canonical layout until the pairs are interleaved by block
-    sp.same = ish == jsh;
-    sp.la = sh.sl[a];
-    sp.lb = sh.sl[b];
+    sp.flags = (ish == jsh ? 1 : 0) | sh.sl[a] << 8 | sh.sl[b] << 16;
     sp.a_off = sh.soff[a];
     sp.b_off = sh.soff[b];
     const double* A = sh.centers + 3 * sh.scen[a];
@@ -63,8 +61,10 @@ __global__ void k_build_pairs(const ShellsDev sh, int npairs, const int* __restr
     for (int k = 0; k < 3; ++k) {
         sp.AB[k] = __dsub_rn(A[k], B[k]);
         sp.ABf[k] = (float)sp.AB[k];
-        sp.ABl[k] = (float)(sp.AB[k] - (double)sp.ABf[k]);
     }
+    sp.ABl0 = (float)(sp.AB[0] - (double)sp.ABf[0]);
+    sp.ABl1 = (float)(sp.AB[1] - (double)sp.ABf[1]);
+    sp.ABl2 = (float)(sp.AB[2] - (double)sp.ABf[2]);
     const double ab2 = __dadd_rn(__dadd_rn(__dmul_rn(sp.AB[0], sp.AB[0]), __dmul_rn(sp.AB[1], sp.AB[1])),
                                  __dmul_rn(sp.AB[2], sp.AB[2]));
     const int p0 = poff[c];
@@ -73,10 +73,10 @@ __global__ void k_build_pairs(const ShellsDev sh, int npairs, const int* __restr
     int m = p0;
     for (int i = 0; i < na; ++i) {
         const double ai = sh.alpha[sh.sprim[a] + i], ci = sh.coef[sh.sprim[a] + i];
-        const int jend = sp.same ? i + 1 : nb;
+        const int jend = sp.same() ? i + 1 : nb;
         for (int j = 0; j < jend; ++j, ++m) {
             const double bj = sh.alpha[sh.sprim[b] + j], cj = sh.coef[sh.sprim[b] + j];
-            const double f = (sp.same && i != j) ? 2.0 : 1.0;
+            const double f = (sp.same() && i != j) ? 2.0 : 1.0;
             PrimPair pp;
             pp.p = __dadd_rn(ai, bj);
             pp.rp = 1.0 / pp.p;

@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(128) store_records_kernel(const FockArgs A, co
                         if constexpr (!UNIT_NORMS) v *= nt.v[LA][ia] * nt.v[LB][ib] * nt.v[LC][ic] * nt.v[LD][id];
                         if (!above_cut(v, A.thr_int)) continue;  // TwoElectronInts.cpp:668
                         int i, j, k, l;
-                        if (!canonical_label(bra.a_off + ia, bra.b_off + ib, ket.a_off + ic, ket.b_off + id, bra.same, ket.same,
+                        if (!canonical_label(bra.a_off + ia, bra.b_off + ib, ket.a_off + ic, ket.b_off + id, bra.same(), ket.same(),
                                              bi == ki, i, j, k, l))
                             continue;
                         if (pass == 0) ++n;
