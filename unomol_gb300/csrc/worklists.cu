@@ -66,25 +66,31 @@ __global__ void split_rows(const ShellPair* __restrict__ pairs, const BlockPair*
     mseg[t] = n64;
 }
 
-// Exclusive scan of the two row counts within every block pair (one CUDA block per block pair).
-__global__ void __launch_bounds__(1024) scan_rows(const BlockPair* __restrict__ bps, const long long* __restrict__ c64,
+// Exclusive scan of the two row counts within every block pair (one CTA per block pair).  Each thread takes
+// SCAN_ROWS consecutive rows of a round: the rounds' barriers, not the bytes, are what it spends its time on
+// (32 waters: one row per thread 22 us).
+constexpr int SCAN_ROWS = 8;
+__global__ void __launch_bounds__(512) scan_rows(const BlockPair* __restrict__ bps, const long long* __restrict__ c64,
                                                   const long long* __restrict__ c32, long long* __restrict__ p64,
                                                   long long* __restrict__ p32, long long* __restrict__ n64,
                                                   long long* __restrict__ n32) {
-    __shared__ long long warp_a[32], warp_b[32];
-    __shared__ long long run_a, run_b;
+    __shared__ long long warp_a[2][16], warp_b[2][16];
     const BlockPair bp = bps[blockIdx.x];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (threadIdx.x == 0) {
-        run_a = 0;
-        run_b = 0;
-    }
-    __syncthreads();
-    for (int base = 0; base < bp.bra_count; base += blockDim.x) {
-        const int i = base + threadIdx.x;
-        const long long va = i < bp.bra_count ? c64[bp.prefix_off + i] : 0;
-        const long long vb = i < bp.bra_count ? c32[bp.prefix_off + i] : 0;
-        long long sa = va, sb = vb;  // inclusive warp scan
+    long long run_a = 0, run_b = 0;  // rows of the earlier rounds, in every thread
+    int buf = 0;
+    for (int base = 0; base < bp.bra_count; base += blockDim.x * SCAN_ROWS, buf ^= 1) {
+        const int i0 = base + threadIdx.x * SCAN_ROWS;
+        long long va[SCAN_ROWS], vb[SCAN_ROWS], ta = 0, tb = 0;
+#pragma unroll
+        for (int k = 0; k < SCAN_ROWS; ++k) {
+            const bool in = i0 + k < bp.bra_count;
+            va[k] = in ? c64[bp.prefix_off + i0 + k] : 0;
+            vb[k] = in ? c32[bp.prefix_off + i0 + k] : 0;
+            ta += va[k];
+            tb += vb[k];
+        }
+        long long sa = ta, sb = tb;  // inclusive warp scan of the threads' sums
         for (int o = 1; o < 32; o <<= 1) {
             const long long xa = __shfl_up_sync(0xffffffffu, sa, o), xb = __shfl_up_sync(0xffffffffu, sb, o);
             if (lane >= o) {
@@ -93,37 +99,27 @@ __global__ void __launch_bounds__(1024) scan_rows(const BlockPair* __restrict__ 
             }
         }
         if (lane == 31) {
-            warp_a[wid] = sa;
-            warp_b[wid] = sb;
+            warp_a[buf][wid] = sa;
+            warp_b[buf][wid] = sb;
         }
-        __syncthreads();
-        if (wid == 0) {
-            const int nw = blockDim.x >> 5;
-            long long ta = lane < nw ? warp_a[lane] : 0, tb = lane < nw ? warp_b[lane] : 0;
-            for (int o = 1; o < 32; o <<= 1) {
-                const long long xa = __shfl_up_sync(0xffffffffu, ta, o), xb = __shfl_up_sync(0xffffffffu, tb, o);
-                if (lane >= o) {
-                    ta += xa;
-                    tb += xb;
-                }
+        __syncthreads();  // the other buffer is free for the next round: everyone has read it before this
+        long long ea = run_a + sa - ta, eb = run_b + sb - tb;
+        for (int k = 0; k < (int)(blockDim.x >> 5); ++k) {
+            if (k < wid) {
+                ea += warp_a[buf][k];
+                eb += warp_b[buf][k];
             }
-            if (lane < nw) {
-                warp_a[lane] = ta;  // inclusive sums of the warps
-                warp_b[lane] = tb;
+            run_a += warp_a[buf][k];
+            run_b += warp_b[buf][k];
+        }
+#pragma unroll
+        for (int k = 0; k < SCAN_ROWS; ++k)
+            if (i0 + k < bp.bra_count) {
+                p64[bp.prefix_off + i0 + k] = ea;
+                p32[bp.prefix_off + i0 + k] = eb;
+                ea += va[k];
+                eb += vb[k];
             }
-        }
-        __syncthreads();
-        const long long wa = wid > 0 ? warp_a[wid - 1] : 0, wb = wid > 0 ? warp_b[wid - 1] : 0;
-        if (i < bp.bra_count) {
-            p64[bp.prefix_off + i] = run_a + wa + sa - va;
-            p32[bp.prefix_off + i] = run_b + wb + sb - vb;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            run_a += warp_a[(blockDim.x >> 5) - 1];
-            run_b += warp_b[(blockDim.x >> 5) - 1];
-        }
-        __syncthreads();
     }
     if (threadIdx.x == 0) {
         n64[blockIdx.x] = run_a;
