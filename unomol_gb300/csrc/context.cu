@@ -6,10 +6,9 @@
 // (ab|ab) is computed; pairs are re-sorted by descending bound within their block; then for every pair
 // of blocks the Schwarz "staircase" (bra i keeps the first n_i ket pairs) gives a compact work list per
 // quartet class.  The host keeps the block boundaries and the block-pair list.
-// Fock build (fock_rhf / fock_uhf): expand packed P to a dense N x N copy, zero the accumulators,
-// launch one kernel per quartet class (classes alternating over two streams forked from the build's
-// stream; in the mixed-precision build both parts of a class in one launch), fold G += T + T^T into
-// packed storage.
+// Fock build (fock_rhf / fock_uhf): expand packed P to a dense N x N copy, zero the accumulators, launch the
+// kernels of every quartet class (FP64 parts on a high-priority stream, FP32 or pairs-of-floats parts on two
+// low-priority ones, all forked from the build's stream), fold G += T + T^T into packed storage.
 #include <algorithm>
 #include <climits>
 #include <memory>
@@ -640,22 +639,20 @@ int ensure_density_buffers(UnomolCtx* ctx, bool uhf) {
     return UNOMOL_OK;
 }
 
-// One class launch with the reference's choice of integral method (TwoElectronInts.cpp:658-666): MD
-// for la+lb+lc+ld > 8 and for every class in the MD mode; otherwise Rys, by the templated kernels for
-// the s/p/d classes they cover and by the runtime-L kernel for the rest.
-static cudaError_t launch_class_kernel(const UnomolCtx* ctx, const ClassLaunch& L, bool uhf, bool fp32, const FockArgs& A,
-                                       cudaStream_t s) {
-    const int la = pc_la(L.bc), lb = pc_lb(L.bc), lc = pc_la(L.kc), ld = pc_lb(L.kc);
-    if (ctx->eri_method == UNOMOL_ERI_MD || la + lb + lc + ld > 8) return launch_fock_md(la, lb, lc, ld, uhf, A, ctx->nt, s);
-    if (L.bc < NTMPLCLASS && L.kc < NTMPLCLASS)
-        return fp32 ? launch_fock_fp32(L.bc, L.kc, uhf, A, ctx->nt, ctx->d_rys32, s)
-                    : launch_fock_fp64(L.bc, L.kc, uhf, A, ctx->nt, ctx->d_rys, s);
-    return launch_fock_generic(la, lb, lc, ld, uhf, fp32, A, ctx->nt, ctx->d_rys, ctx->d_rys32, s);
+// The integral method of a class (TwoElectronInts.cpp:658-666): MD for la+lb+lc+ld > 8 and for every class in
+// the MD mode, otherwise Rys.
+static bool class_is_md(const UnomolCtx* ctx, const ClassLaunch& L) {
+    return ctx->eri_method == UNOMOL_ERI_MD || pc_la(L.bc) + pc_lb(L.bc) + pc_la(L.kc) + pc_lb(L.kc) > 8;
 }
 
-// One class of an FP64 build: launches of few quartets in FP64 with a warp per quartet; otherwise the
-// quartets at or above SPLIT_CUT in FP64 on stream sh (a few lanes per quartet) and those below it in pairs
-// of floats on stream sl.  Classes without those kernels (MD, f and g shells, large d classes) as one launch.
+// The FP32 part of one Rys class: the templated kernels for the s/p/d classes, the runtime-L one for the rest.
+static cudaError_t launch_class_fp32(const UnomolCtx* ctx, const ClassLaunch& L, bool uhf, const FockArgs& A, cudaStream_t s) {
+    if (L.bc < NTMPLCLASS && L.kc < NTMPLCLASS) return launch_fock_fp32(L.bc, L.kc, uhf, A, ctx->nt, ctx->d_rys32, s);
+    return launch_fock_generic32(pc_la(L.bc), pc_lb(L.bc), pc_la(L.kc), pc_lb(L.kc), uhf, A, ctx->nt, ctx->d_rys32, s);
+}
+
+// One class of an FP64 build: the quartets at or above SPLIT_CUT in FP64 on stream sh and those below it in
+// pairs of floats on stream sl; MD classes and those without a template as one launch.
 cudaError_t launch_plain_class(const UnomolCtx* ctx, size_t li, bool uhf, FockArgs A, cudaStream_t sh, cudaStream_t sl,
                                int& launches) {
     const ClassLaunch& L = ctx->launches[li];
@@ -664,17 +661,22 @@ cudaError_t launch_plain_class(const UnomolCtx* ctx, size_t li, bool uhf, FockAr
     A.nbp = L.nbp;
     A.nwork = L.nwork;
     A.mode = 0;
-    const int lsum = pc_la(L.bc) + pc_lb(L.bc) + pc_la(L.kc) + pc_lb(L.kc);
-    if (ctx->eri_method == UNOMOL_ERI_MD || lsum > 8 || !fock_split_class(L.bc, L.kc)) {
+    const int la = pc_la(L.bc), lb = pc_lb(L.bc), lc = pc_la(L.kc), ld = pc_lb(L.kc);
+    if (class_is_md(ctx, L)) {
         ++launches;
-        return launch_class_kernel(ctx, L, uhf, false, A, sl);
+        return launch_fock_md(la, lb, lc, ld, uhf, A, ctx->nt, sl);
     }
-    // a warp per quartet up to 32 quartets per SM (one wave of 8 CTAs of 4 warps); above, one lane per quartet
-    // starts to fill the SMs
-    const long long few = (long long)ctx->nsm * 32;
-    if (L.nwork <= few) {
+    if (!fock_split_class(L.bc, L.kc)) {
         ++launches;
-        return launch_fock_fp64_group(L.bc, L.kc, uhf, A, L.nwork, false, 32, ctx->nt, ctx->d_rys, sl);
+        return launch_fock_coop(la, lb, lc, ld, A, ctx->nt, ctx->d_rys, sl);
+    }
+    // lanes per quartet: a warp up to 32 quartets per SM (one wave of 8 CTAs of 4 warps), four lanes in FP64 from
+    // there on and in pairs of floats up to 256, where one lane each begins to fill the SMs
+    const long long few = (long long)ctx->nsm * 32;
+    if (L.nwork <= 4 * ctx->nsm) {
+        // the smallest molecules: one launch in FP64 for both parts (water in STO-3G 0.24 -> 0.17 ms)
+        ++launches;
+        return launch_fock_group(L.bc, L.kc, uhf, A, L.nwork, false, 32, ctx->nt, ctx->d_rys, sl);
     }
     A.dyn_mseg = ctx->d_mseg_hi;
     const long long hi = ctx->total_hi[li], lo = ctx->total_lo[li];
@@ -685,7 +687,7 @@ cudaError_t launch_plain_class(const UnomolCtx* ctx, size_t li, bool uhf, FockAr
         A.dyn_count = ctx->d_cnt_hi + L.bp_begin;
         A.dyn_begin = ctx->d_begin_hi + L.bp_begin;
         A.dyn_total = ctx->d_total_hi + li;
-        e = launch_fock_fp64_group(L.bc, L.kc, uhf, A, hi, true, hi <= few ? 32 : 4, ctx->nt, ctx->d_rys, sh);
+        e = launch_fock_group(L.bc, L.kc, uhf, A, hi, false, hi <= few ? 32 : 4, ctx->nt, ctx->d_rys, sh);
         ++launches;
     }
     if (e == cudaSuccess && lo > 0) {
@@ -694,7 +696,8 @@ cudaError_t launch_plain_class(const UnomolCtx* ctx, size_t li, bool uhf, FockAr
         A.dyn_count = ctx->d_cnt_lo + L.bp_begin;
         A.dyn_begin = ctx->d_begin_lo + L.bp_begin;
         A.dyn_total = ctx->d_total_lo + li;
-        e = launch_fock_df64(L.bc, L.kc, uhf, A, lo, ctx->nt, sl);
+        e = lo <= 8 * few ? launch_fock_group(L.bc, L.kc, uhf, A, lo, true, lo <= few ? 32 : 4, ctx->nt, ctx->d_rys, sl)
+                          : launch_fock_df64(L.bc, L.kc, uhf, A, lo, ctx->nt, sl);
         ++launches;
     }
     return e;
@@ -797,7 +800,6 @@ int fock_device(UnomolCtx* ctx, const double* dPa, const double* dPb, double* dG
     // (or pairs-of-floats) kernels alternating over two low-priority ones, so that one class's last CTAs
     // overlap the next class's first (n-decane UHF 3.54 -> 3.33 ms; 32 waters mixed, full density, 7.65 -> 7.57)
     const bool split = mixed && ctx->fp32_cut > ctx->skip_cut;
-    const bool templ = ctx->eri_method != UNOMOL_ERI_MD;
     cudaStream_t ls[3] = {s, s, s};
     if (!ctx->counting) {
         CU(cudaEventRecord(ctx->fork, s));
@@ -806,11 +808,10 @@ int fock_device(UnomolCtx* ctx, const double* dPa, const double* dPb, double* dG
             CU(cudaStreamWaitEvent(ls[k], ctx->fork, 0));
         }
     }
-    auto launch_class = [&](const ClassLaunch& L, bool fp32) -> cudaError_t {
-        return launch_class_kernel(ctx, L, uhf, fp32, A, ls[fp32 ? 1 : 0]);
-    };
     for (size_t lk = 0; lk < ctx->launches.size(); ++lk) {
-        const size_t li = ctx->reverse_launches ? ctx->launches.size() - 1 - lk : lk;
+        // FP64 builds: the heaviest angular classes first, whose few, long quartets then overlap the rest (four
+        // polarised waters 753 -> 710 us); mixed builds: last (32 waters, full density, 7.57 against 7.77 ms)
+        const size_t li = (ctx->reverse_launches != 0) == mixed ? ctx->launches.size() - 1 - lk : lk;
         const ClassLaunch& L = ctx->launches[li];
         A.bps = ctx->d_bps + L.bp_begin;
         A.prefix = ctx->d_prefix;
@@ -825,38 +826,33 @@ int fock_device(UnomolCtx* ctx, const double* dPa, const double* dPb, double* dG
             A.dyn_count = ctx->d_cnt64 + L.bp_begin;
             A.dyn_begin = ctx->d_begin64 + L.bp_begin;
             A.dyn_total = ctx->d_total64 + li;
-            const int lsum = pc_la(L.bc) + pc_lb(L.bc) + pc_la(L.kc) + pc_lb(L.kc);
-            if (templ && fock_split_class(L.bc, L.kc) && lsum <= 8) {
-                FockArgs A32 = A;
-                A32.mode = 2;
-                A32.dyn_prefix = ctx->d_pre32;
-                A32.dyn_count = ctx->d_cnt32 + L.bp_begin;
-                A32.dyn_begin = ctx->d_begin32 + L.bp_begin;
-                A32.dyn_total = ctx->d_total32 + li;
-                A32.counter_base += ncls * 32;
+            const int la = pc_la(L.bc), lb = pc_lb(L.bc), lc = pc_la(L.kc), ld = pc_lb(L.kc);
+            const bool md = class_is_md(ctx, L);
+            FockArgs A32 = A;
+            A32.mode = 2;
+            A32.dyn_prefix = ctx->d_pre32;
+            A32.dyn_count = ctx->d_cnt32 + L.bp_begin;
+            A32.dyn_begin = ctx->d_begin32 + L.bp_begin;
+            A32.dyn_total = ctx->d_total32 + li;
+            A32.counter_base += ncls * 32;
+            cudaStream_t s32 = ls[1 + (lk & 1)];
+            if (md) {
+                CU(launch_fock_md(la, lb, lc, ld, uhf, A, ctx->nt, ls[0]));
+                ++launches;
+            } else if (fock_split_class(L.bc, L.kc)) {
                 // the FP64 part (four lanes per quartet), its quartets below SPLIT_CUT (pairs of floats) and the
                 // FP32 part as kernels of their own register counts
                 CU(launch_fock_fp64_part(L.bc, L.kc, uhf, A, A32, ctx->nt, ctx->d_rys, ctx->d_rys32, ctx->nsm * 4, ls[0]));
                 CU(launch_fock_df64_part(L.bc, L.kc, uhf, A, ctx->nt, ctx->nsm * 8, ls[0]));
                 launches += 2;
-                if (split) {
-                    CU(launch_class_kernel(ctx, L, uhf, true, A32, ls[1 + (lk & 1)]));
-                    ++launches;
-                }
-                continue;
-            }
-            CU(launch_class(L, false));
-            if (ctx->fp32_cut > ctx->skip_cut) {
-                A.mode = 2;
-                A.dyn_prefix = ctx->d_pre32;
-                A.dyn_count = ctx->d_cnt32 + L.bp_begin;
-                A.dyn_begin = ctx->d_begin32 + L.bp_begin;
-                A.dyn_total = ctx->d_total32 + li;
-                A.counter_base += ncls * 32;
-                CU(launch_class(L, true));
+            } else {
+                CU(launch_fock_coop(la, lb, lc, ld, A, ctx->nt, ctx->d_rys, ls[0]));
                 ++launches;
             }
-            ++launches;
+            if (split) {
+                CU(md ? launch_fock_md(la, lb, lc, ld, uhf, A32, ctx->nt, s32) : launch_class_fp32(ctx, L, uhf, A32, s32));
+                ++launches;
+            }
         }
     }
     if (ls[0] != s) {  // join the two parts back into the build's stream

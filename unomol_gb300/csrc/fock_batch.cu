@@ -22,28 +22,22 @@ using namespace ugb;
 
 namespace {
 
-template <int BC, int KC, typename R>
-cudaError_t persistent_one(const FockArgs& A, const NormTable& nt, const R* rys, int grid, int block, cudaStream_t s) {
+template <int BC, int KC>
+cudaError_t persistent_one(const FockArgs& A, const NormTable& nt, const float* rys, int grid, int block, cudaStream_t s) {
     constexpr int LA = pc_la(BC), LB = pc_lb(BC), LC = pc_la(KC), LD = pc_lb(KC);
-    if constexpr (QClass<LA, LB, LC, LD>::NF <= 81) {
-        if constexpr (sizeof(R) == 8) return cudaErrorInvalidValue;  // the split build's kernels
-        else fock_jk_persistent<LA, LB, LC, LD, false, R><<<grid, block, 0, s>>>(A, nt, rys);
-    } else if constexpr (sizeof(R) == 8) {
-        // large classes: one item per thread over the whole launch
-        fock_jk_generic<false, double, PrimPair><<<(unsigned)((A.nwork + 63) / 64), 64, 0, s>>>(A, nt, rys, A.prims, LA, LB, LC, LD);
-    } else {
+    if constexpr (QClass<LA, LB, LC, LD>::NF <= 81)
+        fock_jk_persistent<LA, LB, LC, LD, false, float><<<grid, block, 0, s>>>(A, nt, rys);
+    else  // large classes: one item per thread over the whole launch
         fock_jk_generic<false, float, PrimPair32><<<(unsigned)((A.nwork + 63) / 64), 64, 0, s>>>(A, nt, rys, A.prims32, LA, LB, LC, LD);
-    }
     return cudaGetLastError();
 }
 
 #define UGB_CASE(BC, KC) \
     case (BC) * 8 + (KC): \
-        return persistent_one<BC, KC, R>(A, nt, rys, grid, block, s);
+        return persistent_one<BC, KC>(A, nt, rys, grid, block, s);
 
-// FP64 (R = double, FP64 tables) or FP32 (R = float, FP32 tables) persistent launch of one class
-template <typename R>
-cudaError_t launch_persistent(int bc, int kc, const FockArgs& A, const NormTable& nt, const R* rys, int grid,
+// FP32 persistent launch of one class
+cudaError_t launch_persistent(int bc, int kc, const FockArgs& A, const NormTable& nt, const float* rys, int grid,
                               int block, cudaStream_t s) {
     switch (bc * 8 + kc) {
 #include "fock_cases.inc"
@@ -220,15 +214,15 @@ FockArgs split_args(UnomolBatch* b, const BLaunch& L, int k, bool above) {
 }
 
 // One class of the FP64 build: the quartets at or above SPLIT_CUT in FP64 on s0, the others in pairs of
-// floats (persistent tiles) on s1; the large d classes as one launch.
+// floats (persistent tiles) on s1; the large d classes with a warp per quartet.
 cudaError_t batch_plain_class(UnomolBatch* b, const BLaunch& L, int k, cudaStream_t s0, cudaStream_t s1) {
     if (!fock_split_class(L.bc, L.kc))
-        return launch_persistent(L.bc, L.kc, batch_args(b, L, k), b->nt, b->rys, b->nsm * L.ctas_per_sm, L.block, s0);
+        return launch_fock_coop(pc_la(L.bc), pc_lb(L.bc), pc_la(L.kc), pc_lb(L.kc), batch_args(b, L, k), b->nt, b->rys, s1);
     cudaError_t e = cudaSuccess;
     const long long hi = b->total_hi[k], lo = b->total_lo[k];
     if (hi > 0)
-        e = launch_fock_fp64_group(L.bc, L.kc, false, split_args(b, L, k, true), hi, true, hi <= (long long)b->nsm * 32 ? 32 : 4,
-                                   b->nt, b->rys, s0);
+        e = launch_fock_group(L.bc, L.kc, false, split_args(b, L, k, true), hi, false, hi <= (long long)b->nsm * 32 ? 32 : 4, b->nt,
+                              b->rys, s0);
     if (e == cudaSuccess && lo > 0)
         e = launch_fock_df64_persistent(L.bc, L.kc, split_args(b, L, k, false), b->nt, b->nsm * L.ctas_per_sm, L.block, s1);
     return e;
@@ -282,30 +276,21 @@ int batch_build(UnomolBatch* b, cudaStream_t s) {
         // as for one molecule: the FP64 part (four lanes per quartet), its quartets below SPLIT_CUT (pairs of
         // floats) and the FP32 part (persistent) as kernels of their own, classes alternating over the streams
         // (the light classes' two parts in one launch of alternating CTAs: 31.4 against 30.9 ms)
+        FockArgs A32 = A;
+        A32.mode = 2;
+        A32.dyn_prefix = b->d_pre32;
+        A32.dyn_count = b->d_cnt32 + L.bp_begin;
+        A32.dyn_begin = b->d_begin32 + L.bp_begin;
+        A32.dyn_total = b->d_total32 + k;
+        A32.tile_counter = b->d_tiles + 2 * k + 1;
         if (fock_split_class(L.bc, L.kc)) {
-            FockArgs A32 = A;
-            A32.mode = 2;
-            A32.dyn_prefix = b->d_pre32;
-            A32.dyn_count = b->d_cnt32 + L.bp_begin;
-            A32.dyn_begin = b->d_begin32 + L.bp_begin;
-            A32.dyn_total = b->d_total32 + k;
             BCU(launch_fock_fp64_part(L.bc, L.kc, false, A, A32, b->nt, b->rys, b->rys32, b->nsm * 8, ls[k & 1]));
             BCU(launch_fock_df64_part(L.bc, L.kc, false, A, b->nt, b->nsm * 16, ls[k & 1]));
-            A32.tile_counter = b->d_tiles + 2 * k + 1;
-            if (split)
-                BCU(launch_persistent(L.bc, L.kc, A32, b->nt, b->rys32, b->nsm * L.ctas_per_sm, L.block, ls[(k + 1) & 1]));
-            continue;
+        } else {
+            BCU(launch_fock_coop(pc_la(L.bc), pc_lb(L.bc), pc_la(L.kc), pc_lb(L.kc), A, b->nt, b->rys, ls[k & 1]));
         }
-        BCU(launch_persistent(L.bc, L.kc, A, b->nt, b->rys, b->nsm * L.ctas_per_sm, L.block, ls[0]));
-        if (b->fp32_cut > b->skip_cut) {
-            A.mode = 2;  // FP32 part
-            A.dyn_prefix = b->d_pre32;
-            A.dyn_count = b->d_cnt32 + L.bp_begin;
-            A.dyn_begin = b->d_begin32 + L.bp_begin;
-            A.dyn_total = b->d_total32 + k;
-            A.tile_counter = b->d_tiles + 2 * k + 1;
-            BCU(launch_persistent(L.bc, L.kc, A, b->nt, b->rys32, b->nsm * L.ctas_per_sm, L.block, ls[1]));
-        }
+        if (split)
+            BCU(launch_persistent(L.bc, L.kc, A32, b->nt, b->rys32, b->nsm * L.ctas_per_sm, L.block, ls[(k + 1) & 1]));
     }
     if (ls[0] != s)
         for (int q = 0; q < 2; ++q) {
@@ -697,7 +682,7 @@ int unomol_gpu_batch_autotune(UnomolBatch* b, int reps, int* chosen) {
                     if (fock_split_class(L.bc, L.kc))
                         BCU(launch_fock_df64_persistent(L.bc, L.kc, split_args(b, L, (int)k, false), b->nt, b->nsm * c, blk, s));
                     else
-                        BCU(launch_persistent(L.bc, L.kc, batch_args(b, L, (int)k), b->nt, b->rys, b->nsm * c, blk, s));
+                        BCU(batch_plain_class(b, L, (int)k, s, s));
                     BCU(cudaEventRecord(e1, s));
                     BCU(cudaEventSynchronize(e1));
                     float ms = 0.f;

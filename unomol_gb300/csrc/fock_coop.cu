@@ -1,0 +1,36 @@
+// Launches of the warp-per-quartet kernels (fock_coop.cuh).
+#include "fock_coop.cuh"
+#include "fock_dispatch.cuh"
+
+namespace ugb {
+namespace {
+
+template <int KF>
+cudaError_t launch(const FockArgs& A, const NormTable& nt, const double* rys, const CoopShape& q, cudaStream_t s) {
+    const size_t bytes = sizeof(double) * (q.per_cta + (size_t)COOP_WARPS * q.per_warp);
+    if (bytes > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(fock_jk_coop<KF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        if (e != cudaSuccess) return e;
+    }
+    fock_jk_coop<KF><<<(unsigned)((A.nwork + COOP_WARPS - 1) / COOP_WARPS), 32 * COOP_WARPS, bytes, s>>>(A, nt, rys, q.la, q.lb,
+                                                                                                     q.lc, q.ld);
+    return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t launch_fock_coop(int la, int lb, int lc, int ld, const FockArgs& A, const NormTable& nt, const double* rys,
+                             cudaStream_t s) {
+    if (A.nwork <= 0) return cudaSuccess;
+    const CoopShape q(la, lb, lc, ld);
+    if (la + lb + lc + ld > 8) return cudaErrorInvalidValue;
+    // function quartets per lane: the next of a few register budgets
+    if (q.nf <= 4 * 32) return launch<4>(A, nt, rys, q, s);
+    if (q.nf <= 7 * 32) return launch<7>(A, nt, rys, q, s);
+    if (q.nf <= 12 * 32) return launch<12>(A, nt, rys, q, s);
+    if (q.nf <= 21 * 32) return launch<21>(A, nt, rys, q, s);
+    if (q.nf <= 41 * 32) return launch<41>(A, nt, rys, q, s);
+    return cudaErrorInvalidValue;
+}
+
+}  // namespace ugb

@@ -1,5 +1,5 @@
-// Kernels of the split FP64 build: the quartets below SPLIT_CUT in pairs of floats, and FP64 kernels with
-// several lanes per quartet for the rest and for launches of few quartets.
+// Kernels of the split FP64 build: the quartets below SPLIT_CUT in pairs of floats, the others in FP64, with
+// several lanes per quartet where they are few.
 #include "fock_df64.cuh"
 #include "fock_dispatch.cuh"
 
@@ -33,18 +33,19 @@ static cudaError_t launch_persist(const FockArgs& A, const NormTable& nt, int gr
 }
 
 template <int BC, int KC, bool UHF>
-static cudaError_t launch_group(const FockArgs& A, long long items, bool dyn, int lanes, const NormTable& nt, const double* rys,
-                                cudaStream_t s) {
+static cudaError_t launch_group(const FockArgs& A, long long items, bool pairs_of_floats, int lanes, const NormTable& nt,
+                                const double* rys, cudaStream_t s) {
     constexpr int LA = pc_la(BC), LB = pc_lb(BC), LC = pc_la(KC), LD = pc_lb(KC);
     if (items <= 0) return cudaSuccess;
     if constexpr (QClass<LA, LB, LC, LD>::NF <= 81) {
         const unsigned blocks = (unsigned)((items * lanes + FOCK_THREADS - 1) / FOCK_THREADS);
         if (lanes == 32) {
-            if (dyn) fock_jk_fp64_group<LA, LB, LC, LD, UHF, 32, true><<<blocks, FOCK_THREADS, 0, s>>>(A, nt, rys);
-            else fock_jk_fp64_group<LA, LB, LC, LD, UHF, 32, false><<<blocks, FOCK_THREADS, 0, s>>>(A, nt, rys);
+            const size_t bytes = sizeof(double) * (FOCK_THREADS / 32) * group_smem<LA, LB, LC, LD>();
+            if (pairs_of_floats) fock_jk_group<LA, LB, LC, LD, UHF, 32, true><<<blocks, FOCK_THREADS, bytes, s>>>(A, nt, rys);
+            else fock_jk_group<LA, LB, LC, LD, UHF, 32, false><<<blocks, FOCK_THREADS, bytes, s>>>(A, nt, rys);
         } else {
-            if (dyn) fock_jk_fp64_group<LA, LB, LC, LD, UHF, 4, true><<<blocks, FOCK_THREADS, 0, s>>>(A, nt, rys);
-            else fock_jk_fp64_group<LA, LB, LC, LD, UHF, 4, false><<<blocks, FOCK_THREADS, 0, s>>>(A, nt, rys);
+            if (pairs_of_floats) fock_jk_group<LA, LB, LC, LD, UHF, 4, true><<<blocks, FOCK_THREADS, 0, s>>>(A, nt, rys);
+            else fock_jk_group<LA, LB, LC, LD, UHF, 4, false><<<blocks, FOCK_THREADS, 0, s>>>(A, nt, rys);
         }
         return cudaGetLastError();
     } else {
@@ -83,11 +84,11 @@ cudaError_t launch_fock_df64_persistent(int bc, int kc, const FockArgs& A, const
 #undef UGB_CASE
 #define UGB_CASE(BC, KC)                                                              \
     case (BC) * 8 + (KC):                                                             \
-        return uhf ? launch_group<BC, KC, true>(A, items, dyn, lanes, nt, rys, stream) \
-                   : launch_group<BC, KC, false>(A, items, dyn, lanes, nt, rys, stream);
+        return uhf ? launch_group<BC, KC, true>(A, items, pairs_of_floats, lanes, nt, rys, stream) \
+                   : launch_group<BC, KC, false>(A, items, pairs_of_floats, lanes, nt, rys, stream);
 
-cudaError_t launch_fock_fp64_group(int bc, int kc, bool uhf, const FockArgs& A, long long items, bool dyn, int lanes,
-                                   const NormTable& nt, const double* rys, cudaStream_t stream) {
+cudaError_t launch_fock_group(int bc, int kc, bool uhf, const FockArgs& A, long long items, bool pairs_of_floats, int lanes,
+                              const NormTable& nt, const double* rys, cudaStream_t stream) {
     switch (bc * 8 + kc) {
 #include "fock_cases.inc"
         default:

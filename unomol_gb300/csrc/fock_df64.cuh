@@ -9,7 +9,7 @@
 // primitive quartet of (ps|ss) is about 65 FP64 instructions (1040 SM clocks per warp) or about 350 FP32
 // ones (88 clocks at full issue).  Here issue is 50-60 % active, the L1 data pipe 50-60 % and the FP64 pipe
 // (the density contraction) 17-33 %, with the loads the leading stall.  One build, GB300: 32 waters 6-31G
-// 78.5 -> 22.3 ms, n-decane cation UHF 12.1 -> 3.5 ms (with the group kernels below).
+// 74.6 -> 21.2 ms, n-decane cation UHF 12.1 -> 2.8 ms (with the group kernels below).
 // Measured beside it: look-ahead for the next surviving primitive quartet (as the FP64 kernels) instead of
 // plain loops, kept for la+lb+lc+ld = 2 only ((ps|ps) 3.9 against 4.2 ms, (ps|ss) 7.6 against 6.9); 64
 // registers for (ss|ss) and (ps|ss) (25.3 -> 24.0 ms for the build).
@@ -52,28 +52,33 @@ __device__ __forceinline__ df df_poly(const float* __restrict__ c, float yh, flo
     return r;
 }
 
+// Interval k and local coordinate y = yh + yl = 2 (T / H - k) - 1 of T.  above: intervals (k H, (k + 1) H],
+// for the two-root tables (the reference's form starts above T = 15 and ends at T = 40); else [k H, (k + 1) H).
+__device__ __forceinline__ int df_index(bool above, df T, float& yh, float& yl) {
+    const float f = 4.0f * T.h;
+    int k;
+    if (above) {
+        const float c = ceilf(f);
+        k = max((int)c - ((c == f && T.l > 0.f) ? 0 : 1), 0);
+    } else {
+        k = max((int)f, 0);
+    }
+    // 8 T - (2 k + 1); the leading part rounds only below T = 1/8
+    const float T8 = 8.0f * T.h, m = float(2 * k + 1);
+    yh = __fsub_rn(T8, m);
+    yl = __fmaf_rn(8.0f, T.l, __fsub_rn(T8, __fadd_rn(yh, m)));
+    return k;
+}
+
 // Rys nodes and weights in double-float; rs_T etc. as rys_roots.  compat: the two-root block with the
 // reference's form in 15 < T <= 40.
 template <int NR, bool NEED_X>
 __device__ __forceinline__ void df_roots(df T, const float* __restrict__ tab, bool compat, df* x, df* w) {
     constexpr float TMAX = float(rys_tmax(NR));
     if (T.h < TMAX) {
-        const float f = 4.0f * T.h;
-        int k;
-        const float* blk = tab + rys_off(NR, DF_STRIDE, RYS_H);
-        if constexpr (NR == 2) {
-            // intervals (k H, (k + 1) H]: the reference's form starts above T = 15 and ends at T = 40
-            const float c = ceilf(f);
-            k = (int)c - ((c == f && T.l > 0.f) ? 0 : 1);
-            k = max(k, 0);
-            if (compat) blk = tab + DF_COMPAT2;
-        } else {
-            k = max((int)f, 0);
-        }
-        // y = 2 (T / H - k) - 1 = 8 T - (2 k + 1); the leading part rounds only below T = 1/8
-        const float T8 = 8.0f * T.h, m = float(2 * k + 1), yh = __fsub_rn(T8, m);
-        const float yl = __fmaf_rn(8.0f, T.l, __fsub_rn(T8, __fadd_rn(yh, m)));
-        blk += k * (2 * NR * DF_STRIDE);
+        float yh, yl;
+        const int k = df_index(NR == 2, T, yh, yl);
+        const float* blk = tab + (NR == 2 && compat ? DF_COMPAT2 : rys_off(NR, DF_STRIDE, RYS_H)) + k * (2 * NR * DF_STRIDE);
 #pragma unroll
         for (int i = 0; i < NR; ++i) {
             if (NEED_X) x[i] = df_poly(blk + 2 * i * DF_STRIDE, yh, yl);
@@ -162,6 +167,14 @@ __device__ __forceinline__ double df_to_f64(df a) {
     return cvt(a.h) + cvt(a.l);
 }
 
+// SRTERM E_ab E_cd / sqrt(p + q) > PRIM_CUT on all 48 bits
+__device__ __forceinline__ bool df_passes(df p, df Eab, df q, df Ecd) {
+    const float sh = float(SRTERM), sl = float(SRTERM - double(float(SRTERM)));
+    const float ch = float(PRIM_CUT), cl = float(PRIM_CUT - double(float(PRIM_CUT)));
+    const df v = df_mul(df_mul({sh, sl}, df_mul(Eab, Ecd)), df_rsqrt(df_add(p, q)));
+    return __fadd_rn(__fsub_rn(v.h, ch), __fsub_rn(v.l, cl)) > 0.f;
+}
+
 __device__ __forceinline__ df pair_ab(const ShellPair& p, int k) {
     return {p.ABf[k], k == 0 ? p.ABl0 : k == 1 ? p.ABl1 : p.ABl2};
 }
@@ -172,7 +185,7 @@ template <int LA, int LB, int LC, int LD>
 __device__ __forceinline__ void shell_quartet_df64(const ShellPair& bra, const ShellPair& ket,
                                                    const PrimPairDF* __restrict__ prims, const float* __restrict__ tab,
                                                    float prim_cut32, bool compat, df (&acc)[QClass<LA, LB, LC, LD>::NF],
-                                                   unsigned* npass) {
+                                                   unsigned* npass, int part = 0, int nparts = 1) {
     using Q = QClass<LA, LB, LC, LD>;
     constexpr int NR = Q::NR;
     constexpr int L12 = LA + LB, L34 = LC + LD;
@@ -186,12 +199,7 @@ __device__ __forceinline__ void shell_quartet_df64(const ShellPair& bra, const S
     auto passes = [&](const df& bp_p, const df& bp_E, const df& kp_p, const df& kp_E) {
         const float v32 = float(SRTERM) * bp_E.h * kp_E.h * rsqrtf(bp_p.h + kp_p.h);
         if (v32 < lo32) return false;
-        if (v32 <= hi32) {
-            const float sh = float(SRTERM), sl = float(SRTERM - double(float(SRTERM)));
-            const float ch = float(PRIM_CUT), cl = float(PRIM_CUT - double(float(PRIM_CUT)));
-            const df v = df_mul(df_mul({sh, sl}, df_mul(bp_E, kp_E)), df_rsqrt(df_add(bp_p, kp_p)));
-            if (!(__fadd_rn(__fsub_rn(v.h, ch), __fsub_rn(v.l, cl)) > 0.f)) return false;
-        }
+        if (v32 <= hi32 && !df_passes(bp_p, bp_E, kp_p, kp_E)) return false;
         return true;
     };
     auto primitive = [&](const PrimPairDF& bp, const PrimPairDF& kp) {
@@ -247,6 +255,15 @@ __device__ __forceinline__ void shell_quartet_df64(const ShellPair& bra, const S
             }
         }
     };
+    if (nparts > 1) {  // the caller's lanes split the quartet (as shell_quartet_eri)
+        for (int t = part; t < nb * nk; t += nparts) {
+            const int ib = t / nk, ik = t - ib * nk;
+            const PrimPairDF bp = pb[ib * sb];
+            const PrimPairDF kp = pk[ik * sk];
+            if (passes(bp.p, bp.E, kp.p, kp.E)) primitive(bp, kp);
+        }
+        return;
+    }
     if constexpr (L12 + L34 == 2) {
         int ib = 0, ik = 0, cb = -1;
         float rowf = 0.f;  // bound of SRTERM E_ab / sqrt(p + q) over the kets
@@ -338,20 +355,105 @@ __global__ void __launch_bounds__(256, LA + LB + LC + LD <= 1 ? 4 : 1) fock_jk_d
     }
 }
 
-// FP64 integrals with NP lanes per shell quartet, each summing every NP-th primitive quartet: where a launch
-// holds few quartets, one lane each leaves the GPU idle behind a serial chain of primitive quartets (water in
-// STO-3G, 81 of them per quartet: 1.36 -> 0.17 ms per build with a warp each).  DYN: the quartets of a split
-// list (those at or above SPLIT_CUT: few, and the costliest of the build); otherwise every quartet of the class.
-template <int LA, int LB, int LC, int LD, bool UHF, int NP, bool DYN>
-__global__ void __launch_bounds__(128) fock_jk_fp64_group(const FockArgs A, const NormTable nt, const double* __restrict__ rys) {
+// Sums of the 32 lanes' acc[0..N), scattered: the lane ends with the sums of elements first .. first + count - 1
+// in acc[0 ..].  Halving exchanges: in each the lane keeps one half of its elements and adds its partner's.
+__device__ __forceinline__ double sum_exchange(double keep, double send, int o) {
+    return keep + __shfl_xor_sync(0xffffffffu, send, o);
+}
+__device__ __forceinline__ df sum_exchange(df keep, df send, int o) {
+    return df_add(keep, {__shfl_xor_sync(0xffffffffu, send.h, o), __shfl_xor_sync(0xffffffffu, send.l, o)});
+}
+template <int N, int O, class T, int M>
+__device__ __forceinline__ void reduce_scatter(T (&acc)[M], int& first, int& count) {
+    constexpr int H = (N + 1) / 2;
+    const bool upper = threadIdx.x & O;
+#pragma unroll
+    for (int i = 0; i < H; ++i) {
+        const T lo = acc[i], hi = i + H < N ? acc[i + H < N ? i + H : 0] : T{};
+        acc[i] = sum_exchange(upper ? hi : lo, upper ? lo : hi, O);
+    }
+    first += upper ? H : 0;
+    count = upper ? max(count - H, 0) : min(count, H);
+    if constexpr (O > 1) reduce_scatter<H, O / 2>(acc, first, count);
+}
+__host__ __device__ constexpr int scatter_left(int n) {  // elements per lane after the five exchanges
+    for (int k = 0; k < 5; ++k) n = (n + 1) / 2;
+    return n;
+}
+// Shared memory of the contraction by a warp, in doubles: the integrals (odd row stride) and the density blocks.
+template <int LA, int LB, int LC, int LD>
+__host__ __device__ constexpr int group_smem() {
+    using Q = QClass<LA, LB, LC, LD>;
+    return Q::NA * Q::NB * ((Q::NC * Q::ND) | 1) + Q::NA * Q::NB + Q::NC * Q::ND + (Q::NA + Q::NB) * (Q::NC + Q::ND);
+}
+
+// One quartet of a split list (or, mode 0, of the class's whole list) on NP lanes, each summing every NP-th primitive quartet: where a launch holds few
+// quartets, one lane each leaves the GPU idle behind a serial chain of primitive quartets (water in STO-3G, 81
+// of them per quartet: 1.36 -> 0.17 ms per build with a warp each).  DF: in pairs of floats (below SPLIT_CUT),
+// otherwise in FP64 (the others: few, and the costliest of the build).
+template <int LA, int LB, int LC, int LD, bool UHF, int NP, bool DF>
+__global__ void __launch_bounds__(128) fock_jk_group(const FockArgs A, const NormTable nt, const double* __restrict__ rys) {
+    using Q = QClass<LA, LB, LC, LD>;
     const int lane = threadIdx.x & 31, sub = lane / NP, part = lane % NP;
     const unsigned gmask = NP == 32 ? 0xffffffffu : ((1u << (NP & 31)) - 1u) << (sub * NP);
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     int bi, ki;
-    if (!decode_warp_items<DYN>(A, warp * (32 / NP), sub, bi, ki)) return;  // uniform over a group
+    const long long g0 = warp * (32 / NP);
+    if (!(A.mode == 0 ? decode_warp_items<false>(A, g0, sub, bi, ki) : decode_warp_items<true>(A, g0, sub, bi, ki))) return;
     const ShellPair bra = A.pairs[bi];
     const ShellPair ket = A.pairs[ki];
-    quartet_item_group<LA, LB, LC, LD, UHF, double, NP>(A, nt, rys, bra, ket, bi == ki, part, gmask);
+    if constexpr (NP == 32) {
+        // the lanes' partial sums scattered over the warp (81 elements: 82 additions per lane, 405 where every lane
+        // gets every sum), then the contraction by all lanes: (pp|pp) of water in STO-3G 112 -> 68 us, four waters
+        // with d shells 1.15 -> 0.75 ms per build
+        extern __shared__ double smem[];
+        constexpr int VS = (Q::NC * Q::ND) | 1;
+        double* V = smem + (threadIdx.x >> 5) * group_smem<LA, LB, LC, LD>();
+        unsigned npass = 0;
+        std::conditional_t<DF, df, double> acc[Q::NF];
+        if constexpr (DF)
+            shell_quartet_df64<LA, LB, LC, LD>(bra, ket, A.primsdf, A.rysdf, A.prim_cut32, A.rys_compat != 0, acc,
+                                               A.counters ? &npass : nullptr, part, NP);
+        else
+            shell_quartet_eri<LA, LB, LC, LD, double, PrimPair>(bra, ket, A.prims, rys, A.prim_cut, A.prim_cut32, A.rys_compat != 0,
+                                                                acc, A.counters ? &npass : nullptr, part, NP);
+        int first = 0, count = Q::NF;
+        reduce_scatter<Q::NF, 16>(acc, first, count);
+        const int ndeg = (bra.same() ? 1 : 0) + (ket.same() ? 1 : 0) + (bi == ki ? 1 : 0);
+        constexpr int LEFT = scatter_left(Q::NF);
+#pragma unroll
+        for (int i = 0; i < LEFT; ++i)
+            if (i < count) {
+                const int f = first + i, ab = f / (Q::NC * Q::ND), cd = f - ab * (Q::NC * Q::ND);
+                double v;
+                if constexpr (DF) v = df_to_f64(acc[i]);
+                else v = acc[i];
+                if constexpr (LA > 1 || LB > 1 || LC > 1 || LD > 1)
+                    v *= nt.v[LA][ab / Q::NB] * nt.v[LB][ab % Q::NB] * nt.v[LC][cd / Q::ND] * nt.v[LD][cd % Q::ND];
+                V[ab * VS + cd] = above_cut(v, A.thr_int) ? scale_pow2(v, -ndeg) : 0.0;
+            }
+        digest_shared(A, bra, ket, V, Q::NA, Q::NB, Q::NC, Q::ND, VS);
+        if (A.counters) count_flush(A, npass);
+    } else if constexpr (!DF) {
+        quartet_item_group<LA, LB, LC, LD, UHF, double, NP>(A, nt, rys, bra, ket, bi == ki, part, gmask);
+    } else {
+        unsigned npass = 0;
+        double v[Q::NF];
+        {
+            df acc[Q::NF];
+            shell_quartet_df64<LA, LB, LC, LD>(bra, ket, A.primsdf, A.rysdf, A.prim_cut32, A.rys_compat != 0, acc,
+                                               A.counters ? &npass : nullptr, part, NP);
+#pragma unroll
+            for (int o = 1; o < NP; o <<= 1)
+#pragma unroll
+                for (int f = 0; f < Q::NF; ++f)
+                    acc[f] = df_add(acc[f], {__shfl_xor_sync(gmask, acc[f].h, o), __shfl_xor_sync(gmask, acc[f].l, o)});
+#pragma unroll
+            for (int f = 0; f < Q::NF; ++f) v[f] = df_to_f64(acc[f]);
+        }
+        if (part == 0) digest_jk<LA, LB, LC, LD, UHF, double>(A, bra, ket, bi == ki, v, nt);
+        if (A.counters) count_flush(A, npass);
+    }
 }
 
 }  // namespace ugb

@@ -1,6 +1,6 @@
 // Launch table of the class-templated Fock kernels.  Pair class c = la(la+1)/2 + lb (la >= lb);
-// quartet classes are (bra class >= ket class).  One translation unit per arithmetic type
-// instantiates all of them (fock_fp64.cu, fock_fp32.cu).
+// quartet classes are (bra class >= ket class).  One translation unit per kind of kernel instantiates all of
+// them.
 #pragma once
 #include <vector>
 
@@ -13,10 +13,7 @@ struct NormTable;
 __host__ __device__ constexpr int pc_la(int c) { return (c >= 1) + (c >= 3) + (c >= 6) + (c >= 10); }
 __host__ __device__ constexpr int pc_lb(int c) { return c - pc_la(c) * (pc_la(c) + 1) / 2; }
 
-// Launches the Fock kernel of quartet class (bc | kc) over `A.nwork` work items on `stream`.
-// Returns cudaSuccess or the launch error.  FP64: the classes that fock_split_class does not accept.
-cudaError_t launch_fock_fp64(int bc, int kc, bool uhf, const FockArgs& A, const NormTable& nt,
-                             const double* rys, cudaStream_t stream);
+// The FP32 Fock kernel of quartet class (bc | kc) over `A.nwork` work items on `stream`.
 cudaError_t launch_fock_fp32(int bc, int kc, bool uhf, const FockArgs& A, const NormTable& nt,
                              const float* rys, cudaStream_t stream);
 // Whether a class has the templated kernels of the split builds (s, p and d shells, at most 81 function
@@ -38,15 +35,19 @@ cudaError_t launch_fock_df64(int bc, int kc, bool uhf, const FockArgs& A, long l
 // The same over a fixed grid pulling tiles of `block` quartets (RHF; batches of molecules).
 cudaError_t launch_fock_df64_persistent(int bc, int kc, const FockArgs& A, const NormTable& nt, int grid, int block,
                                         cudaStream_t stream);
-// One class in FP64 with `lanes` (4 or 32) lanes per quartet: `items` of a split list (dyn) or of the whole class.
-cudaError_t launch_fock_fp64_group(int bc, int kc, bool uhf, const FockArgs& A, long long items, bool dyn, int lanes,
-                                   const NormTable& nt, const double* rys, cudaStream_t stream);
+// `items` of a split list, in FP64 or in pairs of floats, with `lanes` (4 or 32) lanes per quartet.
+cudaError_t launch_fock_group(int bc, int kc, bool uhf, const FockArgs& A, long long items, bool pairs_of_floats, int lanes,
+                              const NormTable& nt, const double* rys, cudaStream_t stream);
 // All for the classes that fock_split_class accepts.  The root tables of the first:
 std::vector<float> df_rys_tables();
 
-// Runtime-L Rys kernel (classes with f or g shells and la+lb+lc+ld <= 8), FP64 or FP32.
-cudaError_t launch_fock_generic(int la, int lb, int lc, int ld, bool uhf, bool fp32, const FockArgs& A,
-                                const NormTable& nt, const double* rys, const float* rys32, cudaStream_t stream);
+// The Rys classes that fock_split_class does not accept (la+lb+lc+ld <= 8), one warp per quartet (fock_coop.cuh):
+// over A's work list in FP64.  RHF or UHF by A.Pb.
+cudaError_t launch_fock_coop(int la, int lb, int lc, int ld, const FockArgs& A, const NormTable& nt, const double* rys,
+                             cudaStream_t stream);
+// Runtime-L Rys kernel of the same classes' FP32 part, one lane per quartet.
+cudaError_t launch_fock_generic32(int la, int lb, int lc, int ld, bool uhf, const FockArgs& A, const NormTable& nt,
+                                  const float* rys32, cudaStream_t stream);
 // McMurchie-Davidson kernel (la+lb+lc+ld > 8, or every class in the MD mode), FP64.
 cudaError_t launch_fock_md(int la, int lb, int lc, int ld, bool uhf, const FockArgs& A, const NormTable& nt,
                            cudaStream_t stream);

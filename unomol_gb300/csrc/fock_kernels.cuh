@@ -722,6 +722,83 @@ __device__ __forceinline__ void digest_jk(const FockArgs& A, const ShellPair& br
     }
 }
 
+// Density contraction and scatter of one shell quartet by a whole warp (all 32 lanes call it), output by output:
+// V[ab * vs + cd] holds the integrals in shared memory (normalised, cut, with the degeneracy factor of digest_jk),
+// followed by room for the six density blocks; one lane per element of J or K, one atomic each.  RHF or UHF by A.Pb.
+__device__ __forceinline__ void digest_shared(const FockArgs& A, const ShellPair& bra, const ShellPair& ket, double* V, int na,
+                                              int nb, int nc, int nd, int vs) {
+    const int lane = threadIdx.x & 31, nab = na * nb, ncd = nc * nd;
+    int N = A.nbf;
+    long long off = 0;
+    if (A.mol_nbf) {
+        N = A.mol_nbf[bra.pad];
+        off = A.mol_base[bra.pad];
+    }
+    double* Pab = V + nab * vs;
+    double* Pcd = Pab + nab;
+    double* Pac = Pcd + ncd;
+    double* Pad = Pac + na * nc;
+    double* Pbc = Pad + na * nd;
+    double* Pbd = Pbc + nb * nc;
+    const int a0 = bra.a_off, b0 = bra.b_off, c0 = ket.a_off, d0 = ket.b_off;
+    const bool uhf = A.Pb != nullptr;
+    const double jf = uhf ? 2.0 : 4.0;
+    for (int spin = 0; spin < (uhf ? 2 : 1); ++spin) {
+        const double* __restrict__ P = (spin ? A.Pb : A.Pa) + off;
+        double* __restrict__ T = (spin ? A.Tb : A.Ta) + off;
+        auto block = [&](double* dst, int r0, int nrow, int col0, int ncol) {
+            for (int e = lane; e < nrow * ncol; e += 32) dst[e] = __ldg(P + (long long)(r0 + e / ncol) * N + col0 + e % ncol);
+        };
+        __syncwarp();
+        if (spin == 0) {
+            block(Pab, a0, na, b0, nb);
+            block(Pcd, c0, nc, d0, nd);
+            if (uhf) {  // the Coulomb part takes the total density
+                for (int e = lane; e < nab; e += 32) Pab[e] += __ldg(A.Pb + off + (long long)(a0 + e / nb) * N + b0 + e % nb);
+                for (int e = lane; e < ncd; e += 32) Pcd[e] += __ldg(A.Pb + off + (long long)(c0 + e / nd) * N + d0 + e % nd);
+            }
+        }
+        block(Pac, a0, na, c0, nc);
+        block(Pad, a0, na, d0, nd);
+        block(Pbc, b0, nb, c0, nc);
+        block(Pbd, b0, nb, d0, nd);
+        __syncwarp();
+        if (spin == 0) {
+            for (int e = lane; e < nab; e += 32) {
+                double s = 0.0;
+                for (int k = 0; k < ncd; ++k) s = fma(V[e * vs + k], Pcd[k], s);
+                const long long o = off + (long long)(a0 + e / nb) * N + b0 + e % nb;
+                atomicAdd(A.Ta + o, jf * s);
+                if (uhf) atomicAdd(A.Tb + o, jf * s);
+            }
+            for (int e = lane; e < ncd; e += 32) {
+                double s = 0.0;
+                for (int k = 0; k < nab; ++k) s = fma(V[k * vs + e], Pab[k], s);
+                const long long o = off + (long long)(c0 + e / nd) * N + d0 + e % nd;
+                atomicAdd(A.Ta + o, jf * s);
+                if (uhf) atomicAdd(A.Tb + o, jf * s);
+            }
+        }
+        // K(x, y) -= sum over the other two shells' functions u, w of v D(u, w): x and u from the bra (strides vx,
+        // vu of their index in V's rows), y and w from the ket (vy, vw)
+        auto exchange = [&](int x0, int nx, int vx, int nu, int vu, int y0, int ny, int vy, int nw, int vw, const double* D) {
+            for (int e = lane; e < nx * ny; e += 32) {
+                const int x = e / ny, y = e - x * ny;
+                double s = 0.0;
+                for (int u = 0; u < nu; ++u) {
+                    const double* v = V + (x * vx + u * vu) * vs + y * vy;
+                    for (int k = 0; k < nw; ++k) s = fma(-v[k * vw], D[u * nw + k], s);
+                }
+                atomicAdd(T + (long long)(x0 + x) * N + y0 + y, s);
+            }
+        };
+        exchange(a0, na, nb, nb, 1, c0, nc, nd, nd, 1, Pbd);  // K(a, c)
+        exchange(a0, na, nb, nb, 1, d0, nd, 1, nc, nd, Pbc);  // K(a, d)
+        exchange(b0, nb, 1, na, nb, c0, nc, nd, nd, 1, Pad);  // K(b, c)
+        exchange(b0, nb, 1, na, nb, d0, nd, 1, nc, nd, Pac);  // K(b, d)
+    }
+}
+
 // Optional work counter: primitive quartets past the prefactor cut, summed over the converged lanes of
 // the warp and added to one of 32 slots of the launch (spread to avoid a hot address).
 __device__ __forceinline__ void count_flush(const FockArgs& A, unsigned v) {

@@ -1,4 +1,4 @@
-// Launchers of the classes with f and g shells: runtime-L Rys (la+lb+lc+ld <= 8, FP64 or FP32),
+// Launchers of the classes with f and g shells: runtime-L Rys (la+lb+lc+ld <= 8, FP32),
 // McMurchie-Davidson (la+lb+lc+ld > 8, and every class in the MD mode), and their Schwarz diagonals;
 // the same two methods as record passes of the conventional build (store.cu).
 #include <algorithm>
@@ -9,21 +9,14 @@
 
 namespace ugb {
 
-cudaError_t launch_fock_generic(int la, int lb, int lc, int ld, bool uhf, bool fp32, const FockArgs& A,
-                                const NormTable& nt, const double* rys, const float* rys32, cudaStream_t s) {
+cudaError_t launch_fock_generic32(int la, int lb, int lc, int ld, bool uhf, const FockArgs& A, const NormTable& nt,
+                                  const float* rys32, cudaStream_t s) {
     if (A.nwork <= 0) return cudaSuccess;
     const unsigned blocks = (unsigned)((A.nwork + 63) / 64);
-    if (fp32) {
-        if (uhf)
-            fock_jk_generic<true, float, PrimPair32><<<blocks, 64, 0, s>>>(A, nt, rys32, A.prims32, la, lb, lc, ld);
-        else
-            fock_jk_generic<false, float, PrimPair32><<<blocks, 64, 0, s>>>(A, nt, rys32, A.prims32, la, lb, lc, ld);
-    } else {
-        if (uhf)
-            fock_jk_generic<true, double, PrimPair><<<blocks, 64, 0, s>>>(A, nt, rys, A.prims, la, lb, lc, ld);
-        else
-            fock_jk_generic<false, double, PrimPair><<<blocks, 64, 0, s>>>(A, nt, rys, A.prims, la, lb, lc, ld);
-    }
+    if (uhf)
+        fock_jk_generic<true, float, PrimPair32><<<blocks, 64, 0, s>>>(A, nt, rys32, A.prims32, la, lb, lc, ld);
+    else
+        fock_jk_generic<false, float, PrimPair32><<<blocks, 64, 0, s>>>(A, nt, rys32, A.prims32, la, lb, lc, ld);
     return cudaGetLastError();
 }
 
