@@ -693,7 +693,7 @@ int unomol_guess_predict(UnomolGuess* g, const UnomolBasisDesc* basis, const int
     k_features<<<nblk((long long)nr * g->mlp.n_in_pad), 256, 0, g->s>>>(g->p_rows.p, nr, g->E, g->cfg.n_rbf, g->delta,
                                                                           g->mlp.n_in_pad, g->mlp.X);
     GK(cudaGetLastError());
-    rc = g->mlp.forward_x(nr, g->s);
+    rc = g->mlp.forward_x(nr, g->s, false);
     if (rc) {
         g->err = g->mlp.err;
         return rc;

@@ -73,8 +73,12 @@ cudaError_t tc_gemm_launch(TcGemmArgs g, cudaStream_t s, int num_sms) {
     g.pipeline_polls = g_tc_pipeline_polls.load();
     if ((g.lda & 7) || (g.ldb & 7) || (reinterpret_cast<uintptr_t>(g.A) & 15) || (reinterpret_cast<uintptr_t>(g.B) & 15))
         return cudaErrorInvalidValue;
-    const int bn = g.N <= 64 ? 64 : g.N <= 128 ? 128 : 256;
-    const int tiles_m = (g.M + TC_BM - 1) / TC_BM, tiles_n = (g.N + bn - 1) / bn;
+    // the widest tile that still gives two CTAs per SM: narrower ones share the epilogue (which bounds the network's
+    // shapes) out over more CTAs; a 256-wide tile at 13856 x 256 leaves 109 CTAs (44 us forward, 13 with 64)
+    const int tiles_m = (g.M + TC_BM - 1) / TC_BM;
+    int bn = g.N <= 64 ? 64 : g.N <= 128 ? 128 : 256;
+    while (bn > 64 && (long long)tiles_m * ((g.N + bn - 1) / bn) < 2ll * num_sms) bn /= 2;
+    const int tiles_n = (g.N + bn - 1) / bn;
     const int nk = (g.K + TC_BK - 1) / TC_BK;
     int splits = 1;
     if (g.epi == TC_EPI_F32_ADD) {
@@ -124,11 +128,12 @@ __global__ void k_to_bf16_pad(const float* __restrict__ x, int ldx, int rows, in
     out[t] = __float2bfloat16(c < n_in ? x[(long long)r * ldx + c] : 0.f);
 }
 
-// out[c] += sum_r a[r][c]: one block per 256 rows, one thread per column
+// out[c] += sum_r a[r][c]: one block per COLSUM_ROWS rows, one thread per column
+constexpr int COLSUM_ROWS = 64;
 __global__ void k_colsum(const float* __restrict__ a, int rows, int cols, int lda, float* __restrict__ out) {
     const int c = blockIdx.y * blockDim.x + threadIdx.x;
     if (c >= cols) return;
-    const int r0 = blockIdx.x * 256, r1 = min(rows, r0 + 256);
+    const int r0 = blockIdx.x * COLSUM_ROWS, r1 = min(rows, r0 + COLSUM_ROWS);
     float s = 0.f;
     for (int r = r0; r < r1; ++r) s += a[(long long)r * lda + c];
     atomicAdd(out + c, s);
@@ -182,12 +187,13 @@ uint64_t mix64(uint64_t& s) {
     } while (0)
 
 Mlp::~Mlp() {
-    for (void* p : std::vector<void*>{P, G, Am, Av, Wb, Wt, X, Y, dYb, dZb[0], dZb[1], dZf, Ta, Tb, status})
+    for (void* p : std::vector<void*>{P, G, Am, Av, Wb, Wt, X, Y, dYb, dZb[0], dZb[1], Ta, Tb, status})
         if (p) cudaFree(p);
     for (float* p : Z)
         if (p) cudaFree(p);
-    for (__nv_bfloat16* p : H)
-        if (p) cudaFree(p);
+    for (const auto& v : {H, HT})
+        for (__nv_bfloat16* p : v)
+            if (p) cudaFree(p);
 }
 
 int Mlp::init(int n_in_, int hidden_, int layers_, int n_out_, unsigned long long seed) {
@@ -255,13 +261,15 @@ int Mlp::reserve(int r) {
     auto rel = [](void* p) {
         if (p) cudaFree(p);
     };
-    rel(X), rel(Y), rel(dYb), rel(dZb[0]), rel(dZb[1]), rel(dZf), rel(Ta), rel(Tb);
+    rel(X), rel(Y), rel(dYb), rel(dZb[0]), rel(dZb[1]), rel(Ta), rel(Tb);
     Ta = Tb = nullptr;
     for (float* p : Z) rel(p);
-    for (__nv_bfloat16* p : H) rel(p);
-    X = nullptr, Y = nullptr, dYb = nullptr, dZb[0] = dZb[1] = nullptr, dZf = nullptr;
+    for (const auto& v : {H, HT})
+        for (__nv_bfloat16* p : v) rel(p);
+    X = nullptr, Y = nullptr, dYb = nullptr, dZb[0] = dZb[1] = nullptr;
     Z.assign(layers, nullptr);
     H.assign(layers, nullptr);
+    HT.assign(layers, nullptr);
     cap = 0;
     const size_t R = (size_t)c;
     MLP_CK(cudaMalloc(&X, R * n_in_pad * sizeof(__nv_bfloat16)));
@@ -269,13 +277,13 @@ int Mlp::reserve(int r) {
     MLP_CK(cudaMalloc(&dYb, R * n_out * sizeof(__nv_bfloat16)));
     MLP_CK(cudaMalloc(&dZb[0], R * hidden * sizeof(__nv_bfloat16)));
     MLP_CK(cudaMalloc(&dZb[1], R * hidden * sizeof(__nv_bfloat16)));
-    MLP_CK(cudaMalloc(&dZf, R * hidden * sizeof(float)));
     const size_t Rp = (R + 7) / 8 * 8;  // transposed operands: row stride a multiple of 8 elements
     MLP_CK(cudaMalloc(&Ta, Rp * std::max(hidden, n_out) * sizeof(__nv_bfloat16)));
-    MLP_CK(cudaMalloc(&Tb, Rp * std::max(hidden, n_in_pad) * sizeof(__nv_bfloat16)));
+    MLP_CK(cudaMalloc(&Tb, Rp * n_in_pad * sizeof(__nv_bfloat16)));
     for (int l = 0; l < layers; ++l) {
         MLP_CK(cudaMalloc(&Z[l], R * hidden * sizeof(float)));
         MLP_CK(cudaMalloc(&H[l], R * hidden * sizeof(__nv_bfloat16)));
+        MLP_CK(cudaMalloc(&HT[l], Rp * hidden * sizeof(__nv_bfloat16)));
     }
     cap = c;
     return UNOMOL_OK;
@@ -293,12 +301,13 @@ int Mlp::forward(const float* x, int ldx, int r, cudaStream_t s) {
     return forward_x(r, s);
 }
 
-int Mlp::forward_x(int r, cudaStream_t s) {
+int Mlp::forward_x(int r, cudaStream_t s, bool train) {
     if (r > cap) {
         err = "mlp forward: more rows than reserved";
         return UNOMOL_EINVAL;
     }
     rows = r;
+    have_t = train;
     if (r == 0) return UNOMOL_OK;
     for (int l = 0; l <= layers; ++l) {
         TcGemmArgs g{};
@@ -313,6 +322,7 @@ int Mlp::forward_x(int r, cudaStream_t s) {
         g.status = status;
         if (l < layers) {
             g.epi = TC_EPI_BIAS_SILU;
+            if (train) g.CbT = HT[l], g.ldt = (r + 7) / 8 * 8;
             g.Z = Z[l];
             g.Cb = H[l];
             g.ldc = hidden;
@@ -337,18 +347,21 @@ int Mlp::backward(const float* dy, bool accumulate, cudaStream_t s) {
     const int L = layers;
     k_f32_to_bf16<<<nblk((long long)r * n_out), 256, 0, s>>>(dy, (long long)r * n_out, dYb);
     {
-        dim3 grid(nblk(r), nblk(n_out, 64));
+        dim3 grid(nblk(r, COLSUM_ROWS), nblk(n_out, 64));
         k_colsum<<<grid, 64, 0, s>>>(dy, r, n_out, n_out, G + b_off[L]);
     }
     MLP_CK(cudaGetLastError());
     const int rp = (r + 7) / 8 * 8;
+    if (!have_t) {
+        for (int l = 0; l < L; ++l) MLP_CK(transpose(H[l], r, hidden, hidden, HT[l], rp, s));
+        have_t = true;
+    }
     // dW_L = dY^T . h_L  (operands transposed to K-major: K = rows)
     {
         MLP_CK(transpose(dYb, r, n_out, n_out, Ta, rp, s));
-        MLP_CK(transpose(H[L - 1], r, hidden, hidden, Tb, rp, s));
         TcGemmArgs g{};
         g.A = Ta, g.lda = rp;
-        g.B = Tb, g.ldb = rp;
+        g.B = HT[L - 1], g.ldb = rp;
         g.M = n_out, g.N = hidden, g.K = r;
         g.epi = TC_EPI_F32_ADD, g.Cf = G + w_off[L], g.ldc = din_pad[L];
         g.status = status;
@@ -364,22 +377,16 @@ int Mlp::backward(const float* dy, bool accumulate, cudaStream_t s) {
             g.A = dg, g.lda = dg_ld;
             g.B = Wt + wt_off[l + 1], g.ldb = dout[l + 1];
             g.M = r, g.N = hidden, g.K = dout[l + 1];
-            g.epi = TC_EPI_DSILU, g.Z = Z[l], g.Cb = dZb[cur], g.Cf = dZf, g.ldc = hidden;
+            g.epi = TC_EPI_DSILU, g.Z = Z[l], g.Cb = dZb[cur], g.CbT = Ta, g.ldt = rp, g.colsum = G + b_off[l], g.ldc = hidden;
             g.status = status;
             MLP_CK(tc_gemm_launch(g, s, num_sms));
         }
-        {
-            dim3 grid(nblk(r), nblk(hidden, 256));
-            k_colsum<<<grid, 256, 0, s>>>(dZf, r, hidden, hidden, G + b_off[l]);
-            MLP_CK(cudaGetLastError());
-        }
         // dW_l = dz_l^T . h_l  (h_0 = x; operands transposed to K-major)
         {
-            MLP_CK(transpose(dZb[cur], r, hidden, hidden, Ta, rp, s));
-            MLP_CK(transpose(l == 0 ? X : H[l - 1], r, din_pad[l], din_pad[l], Tb, rp, s));
+            if (l == 0) MLP_CK(transpose(X, r, n_in_pad, n_in_pad, Tb, rp, s));
             TcGemmArgs g{};
             g.A = Ta, g.lda = rp;
-            g.B = Tb, g.ldb = rp;
+            g.B = l == 0 ? Tb : HT[l - 1], g.ldb = rp;
             g.M = hidden, g.N = din_pad[l], g.K = r;
             g.epi = TC_EPI_F32_ADD, g.Cf = G + w_off[l], g.ldc = din_pad[l];
             g.status = status;

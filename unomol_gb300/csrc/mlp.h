@@ -33,7 +33,8 @@ struct Mlp {
     float* Y = nullptr;                        // [cap x n_out]
     __nv_bfloat16* dYb = nullptr;              // [cap x n_out]
     __nv_bfloat16* dZb[2] = {nullptr, nullptr};  // [cap x hidden]
-    float* dZf = nullptr;                      // [cap x hidden]
+    std::vector<__nv_bfloat16*> HT;            // [layers][hidden x rows rounded up to 8]: H transposed, for the weight gradients
+    bool have_t = false;                       // HT belongs to the last forward
     __nv_bfloat16 *Ta = nullptr, *Tb = nullptr;  // transposed operands of the weight gradients
     int* status = nullptr;                     // device flag: a GEMM wait gave up
     std::string err;
@@ -41,8 +42,8 @@ struct Mlp {
     ~Mlp();
     int init(int n_in, int hidden, int layers, int n_out, unsigned long long seed);
     int reserve(int rows);
-    // y = f(x) for rows already written to X (bf16, [rows x n_in_pad], padding zero)
-    int forward_x(int rows, cudaStream_t s);
+    // y = f(x) for rows already written to X (bf16, [rows x n_in_pad], padding zero); train: a backward follows
+    int forward_x(int rows, cudaStream_t s, bool train = true);
     // x from fp32 [rows x ldx], then forward
     int forward(const float* x, int ldx, int rows, cudaStream_t s);
     // G (+)= d loss / d params for the rows of the last forward, dy fp32 [rows x n_out]

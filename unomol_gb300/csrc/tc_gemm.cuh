@@ -37,9 +37,9 @@ constexpr int TC_WAIT_POLLS = 1 << 22;
 
 enum TcEpilogue : int {
     TC_EPI_F32 = 0,         // Cf = acc
-    TC_EPI_BIAS_SILU = 1,   // Z = acc + bias; Cb = silu(Z)
+    TC_EPI_BIAS_SILU = 1,   // Z = acc + bias; Cb = silu(Z), and CbT = its transpose when CbT is set
     TC_EPI_BIAS_F32 = 2,    // Cf = acc + bias
-    TC_EPI_DSILU = 3,       // Cb = acc * silu'(Z), and Cf = the same in fp32 when Cf is set
+    TC_EPI_DSILU = 3,       // Cb = acc * silu'(Z), CbT = its transpose, colsum += its FP32 column sums
     TC_EPI_F32_ADD = 4,     // Cf += acc (atomic; split-K partial tiles)
 };
 
@@ -51,6 +51,9 @@ struct TcGemmArgs {
     const float* bias;       // [N]
     float* Cf;               // fp32 output [M][ldc]
     __nv_bfloat16* Cb;       // bf16 output [M][ldc]
+    __nv_bfloat16* CbT;      // bf16 output transposed [N][ldt] (lanes hold consecutive rows: 64-byte stores)
+    int ldt;
+    float* colsum;           // [N], added to (atomic)
     float* Z;                // fp32 pre-activation out (BIAS_SILU) / in (DSILU), [M][ldc]
     int ldc;
     int chunks_per_split;    // K chunks of one blockIdx.z
@@ -197,15 +200,28 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                      : "memory");
     }
     __syncwarp();
+    const int row = m0 + warp * 32 + lane;
+    const bool in = row < g.M;
+    // the narrow tile's pre-activations, loaded while the MMAs run: the epilogue of a 64-column tile then waits
+    // for no load (the loads of 16 columns at a time, each waited for, made it 68 us at 13856 x 256)
+    constexpr bool PRE = BN == 64;
+    float4 zpre[PRE ? BN / 4 : 1];
+    const bool pre = PRE && g.epi == TC_EPI_DSILU && n0 + BN <= g.N && (g.ldc & 7) == 0;
+    if (PRE && pre && in) {
+#pragma unroll
+        for (int q = 0; q < (PRE ? BN / 4 : 0); ++q)
+            zpre[q] = *reinterpret_cast<const float4*>(g.Z + (long long)row * g.ldc + n0 + 4 * q);
+    }
     const bool ok = mbar_wait(smem_u32(&done), 0);
     if (!ok) atomicExch(&failed, 1);
     asm volatile("tcgen05.fence::after_thread_sync;");
     __syncthreads();
     if (!failed) {
-        const int row = m0 + warp * 32 + lane;
         const bool vec4 = (g.ldc & 3) == 0;
-#pragma unroll 1
+        constexpr int UNR = PRE ? BN / 16 : 1;
+#pragma unroll UNR
         for (int c0 = 0; c0 < BN; c0 += 16) {
+            __syncwarp();  // the load below is warp-wide; lanes past the last row skip the stores above it
             if (n0 + c0 >= g.N) break;  // uniform
             uint32_t r[16];
             const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0;
@@ -215,13 +231,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                 : "r"(taddr));
             asm volatile("tcgen05.wait::ld.sync.aligned;");
-            if (row >= g.M) continue;
             const int col0 = n0 + c0;
             const long long o0 = (long long)row * g.ldc + col0;
             float v[16];
 #pragma unroll
             for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
             const bool full16 = col0 + 16 <= g.N;
+            if (!in && g.epi != TC_EPI_DSILU) continue;
             if (g.epi == TC_EPI_F32 || g.epi == TC_EPI_BIAS_F32) {
                 if (g.epi == TC_EPI_BIAS_F32)
 #pragma unroll
@@ -234,7 +250,15 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                     for (int j = 0; j < 16 && col0 + j < g.N; ++j) g.Cf[o0 + j] = v[j];
                 }
             } else if (g.epi == TC_EPI_F32_ADD) {
-                for (int j = 0; j < 16 && col0 + j < g.N; ++j) atomicAdd(g.Cf + o0 + j, v[j]);
+                if (full16 && vec4 && (reinterpret_cast<uintptr_t>(g.Cf) & 15) == 0) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(g.Cf + o0 + 4 * q), "f"(v[4 * q]),
+                                     "f"(v[4 * q + 1]), "f"(v[4 * q + 2]), "f"(v[4 * q + 3])
+                                     : "memory");
+                } else {
+                    for (int j = 0; j < 16 && col0 + j < g.N; ++j) atomicAdd(g.Cf + o0 + j, v[j]);
+                }
             } else if (g.epi == TC_EPI_BIAS_SILU) {
                 __align__(16) __nv_bfloat16 h[16];
 #pragma unroll
@@ -255,26 +279,54 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                         g.Cb[o0 + j] = h[j];
                     }
                 }
+                if (g.CbT)
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        if (col0 + j < g.N) g.CbT[(long long)(col0 + j) * g.ldt + row] = h[j];
             } else {  // TC_EPI_DSILU
                 __align__(16) __nv_bfloat16 h[16];
+#pragma unroll
                 for (int j = 0; j < 16; ++j) {
-                    const float z = col0 + j < g.N ? g.Z[o0 + j] : 0.f;
+                    float z = 0.f;
+                    if (in) {
+                        if (PRE && pre) {
+                            const float4 q = zpre[PRE ? (c0 + j) / 4 : 0];
+                            z = (j & 3) == 0 ? q.x : (j & 3) == 1 ? q.y : (j & 3) == 2 ? q.z : q.w;
+                        } else if (col0 + j < g.N) {
+                            z = g.Z[o0 + j];
+                        }
+                    }
                     const float s = 1.f / (1.f + __expf(-z));
-                    v[j] = v[j] * s * (1.f + z * (1.f - s));
+                    v[j] = in ? v[j] * s * (1.f + z * (1.f - s)) : 0.f;
                     h[j] = __float2bfloat16(v[j]);
                 }
-                if (full16 && (g.ldc & 7) == 0) {
-                    *reinterpret_cast<uint4*>(g.Cb + o0) = *reinterpret_cast<const uint4*>(h);
-                    *reinterpret_cast<uint4*>(g.Cb + o0 + 8) = *reinterpret_cast<const uint4*>(h + 8);
-                    if (g.Cf)
-#pragma unroll
-                        for (int q = 0; q < 4; ++q)
-                            *reinterpret_cast<float4*>(g.Cf + o0 + 4 * q) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-                } else {
-                    for (int j = 0; j < 16 && col0 + j < g.N; ++j) {
-                        g.Cb[o0 + j] = h[j];
-                        if (g.Cf) g.Cf[o0 + j] = v[j];
+                if (in) {
+                    if (full16 && (g.ldc & 7) == 0) {
+                        *reinterpret_cast<uint4*>(g.Cb + o0) = *reinterpret_cast<const uint4*>(h);
+                        *reinterpret_cast<uint4*>(g.Cb + o0 + 8) = *reinterpret_cast<const uint4*>(h + 8);
+                    } else {
+                        for (int j = 0; j < 16 && col0 + j < g.N; ++j) g.Cb[o0 + j] = h[j];
                     }
+                    if (g.CbT)
+#pragma unroll
+                        for (int j = 0; j < 16; ++j)
+                            if (col0 + j < g.N) g.CbT[(long long)(col0 + j) * g.ldt + row] = h[j];
+                }
+                if (g.colsum) {
+                    // column sums over the warp's 32 rows: halving exchanges leave one column per lane pair
+#pragma unroll
+                    for (int o = 16, n = 8; o > 1; o >>= 1, n >>= 1) {
+                        const bool upper = lane & o;
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            if (j < n) {
+                                const float send = upper ? v[j] : v[j + n], keep = upper ? v[j + n] : v[j];
+                                v[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                            }
+                    }
+                    const float sum = v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+                    const int col = col0 + ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1);
+                    if (!(lane & 1) && col < g.N) atomicAdd(g.colsum + col, sum);
                 }
             }
         }
