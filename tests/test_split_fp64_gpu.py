@@ -50,3 +50,22 @@ def test_split_build_far_from_the_origin(gpu):
     b.centers = b.centers + 4096.0
     H = native.TwoElectronInts(b).form_g(P)
     assert np.abs(G - H).max() <= _bound(b, 1.0) + 3.0 * b.norb ** 2 * 2.0 ** -41
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("basis", ["STO-3G", "6-31G"])
+@pytest.mark.parametrize("system,n", MOLECULES)
+def test_screened_fp64_build_matches_stored_integrals(gpu, system, n, basis):
+    """The density-screened FP64 build with nothing skipped: its part of every class in the group kernels or one
+    lane per quartet, by the number of quartets."""
+    from unomol_gb300 import molecules, native
+    from unomol_gb300.basis import Basis
+    atoms = molecules.water_cluster(n, 5) if system == "water" else molecules.alkane(n)
+    b = Basis(text=molecules.patin_text(atoms, basis))
+    P = rand_density(b.norb, 11)
+    t = native.TwoElectronInts(b)
+    t.set_precision(native.PREC_MIXED, 0.0)
+    t.set_density_screening(0.0)
+    G = t.form_g(P)
+    t.store_integrals(native.STORE_RHF)
+    assert np.abs(G - t.form_g(P)).max() <= _bound(b, np.abs(P).max())

@@ -840,11 +840,10 @@ int fock_device(UnomolCtx* ctx, const double* dPa, const double* dPb, double* dG
                 CU(launch_fock_md(la, lb, lc, ld, uhf, A, ctx->nt, ls[0]));
                 ++launches;
             } else if (fock_split_class(L.bc, L.kc)) {
-                // the FP64 part (four lanes per quartet), its quartets below SPLIT_CUT (pairs of floats) and the
+                // the FP64 part (a few lanes per quartet), its quartets below SPLIT_CUT (pairs of floats) and the
                 // FP32 part as kernels of their own register counts
-                CU(launch_fock_fp64_part(L.bc, L.kc, uhf, A, A32, ctx->nt, ctx->d_rys, ctx->d_rys32, ctx->nsm * 4, ls[0]));
-                CU(launch_fock_df64_part(L.bc, L.kc, uhf, A, ctx->nt, ctx->nsm * 8, ls[0]));
-                launches += 2;
+                CU(launch_mixed_fp64(L.bc, L.kc, uhf, A, A32, ctx->nt, ctx->d_rys, ctx->d_rys32, ctx->nsm, 4, 8, split, ls[0],
+                                     &launches));
             } else {
                 CU(launch_fock_coop(la, lb, lc, ld, A, ctx->nt, ctx->d_rys, ls[0]));
                 ++launches;

@@ -130,6 +130,8 @@ struct FockArgs {
     double thr_int;             // per-integral cut (1e-14)
     double prim_cut;            // primitive prefactor cut (1e-12)
     float thr_int32, prim_cut32, skip_cut32;  // the same cuts in FP32, for the FP32 kernels
+    int only_demoted;           // FP64 part of a mixed build: only its FP32 quartets (the others have a launch of their own)
+    long long df_group_max;     // and up to this many quartets in the part it also takes the pairs-of-floats ones
     float fp32_cut32;           // mixed mode: a quartet with bound * max|P| of its blocks below this runs in FP32
     double fp32_cut;            // mixed mode: bound * max|P| below this -> FP32 part, else FP64 part
     int mode;                   // 0 all quartets; 1 only "large" (FP64 part); 2 only "small" (FP32 part);

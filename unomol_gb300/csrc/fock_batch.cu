@@ -284,8 +284,8 @@ int batch_build(UnomolBatch* b, cudaStream_t s) {
         A32.dyn_total = b->d_total32 + k;
         A32.tile_counter = b->d_tiles + 2 * k + 1;
         if (fock_split_class(L.bc, L.kc)) {
-            BCU(launch_fock_fp64_part(L.bc, L.kc, false, A, A32, b->nt, b->rys, b->rys32, b->nsm * 8, ls[k & 1]));
-            BCU(launch_fock_df64_part(L.bc, L.kc, false, A, b->nt, b->nsm * 16, ls[k & 1]));
+            int nl = 0;
+            BCU(launch_mixed_fp64(L.bc, L.kc, false, A, A32, b->nt, b->rys, b->rys32, b->nsm, 8, 16, split, ls[k & 1], &nl));
         } else {
             BCU(launch_fock_coop(pc_la(L.bc), pc_lb(L.bc), pc_la(L.kc), pc_lb(L.kc), A, b->nt, b->rys, ls[k & 1]));
         }

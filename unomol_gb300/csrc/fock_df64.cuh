@@ -387,6 +387,29 @@ __host__ __device__ constexpr int group_smem() {
     return Q::NA * Q::NB * ((Q::NC * Q::ND) | 1) + Q::NA * Q::NB + Q::NC * Q::ND + (Q::NA + Q::NB) * (Q::NC + Q::ND);
 }
 
+// quartet_item_group (fock_kernels.cuh) in pairs of floats.
+template <int LA, int LB, int LC, int LD, bool UHF, int NP>
+__device__ __forceinline__ void quartet_item_group_df(const FockArgs& A, const NormTable& nt, const ShellPair& bra,
+                                                      const ShellPair& ket, bool same_pair, int part, unsigned gmask) {
+    using Q = QClass<LA, LB, LC, LD>;
+    unsigned npass = 0;
+    double v[Q::NF];
+    {
+        df acc[Q::NF];
+        shell_quartet_df64<LA, LB, LC, LD>(bra, ket, A.primsdf, A.rysdf, A.prim_cut32, A.rys_compat != 0, acc,
+                                           A.counters ? &npass : nullptr, part, NP);
+#pragma unroll
+        for (int o = 1; o < NP; o <<= 1)
+#pragma unroll
+            for (int f = 0; f < Q::NF; ++f)
+                acc[f] = df_add(acc[f], {__shfl_xor_sync(gmask, acc[f].h, o), __shfl_xor_sync(gmask, acc[f].l, o)});
+#pragma unroll
+        for (int f = 0; f < Q::NF; ++f) v[f] = df_to_f64(acc[f]);
+    }
+    if (part == 0) digest_jk<LA, LB, LC, LD, UHF, double>(A, bra, ket, same_pair, v, nt);
+    if (A.counters) count_flush(A, npass);
+}
+
 // One quartet of a split list (or, mode 0, of the class's whole list) on NP lanes, each summing every NP-th primitive quartet: where a launch holds few
 // quartets, one lane each leaves the GPU idle behind a serial chain of primitive quartets (water in STO-3G, 81
 // of them per quartet: 1.36 -> 0.17 ms per build with a warp each).  DF: in pairs of floats (below SPLIT_CUT),
@@ -402,6 +425,11 @@ __global__ void __launch_bounds__(128) fock_jk_group(const FockArgs A, const Nor
     if (!(A.mode == 0 ? decode_warp_items<false>(A, g0, sub, bi, ki) : decode_warp_items<true>(A, g0, sub, bi, ki))) return;
     const ShellPair bra = A.pairs[bi];
     const ShellPair ket = A.pairs[ki];
+    if (A.mode == 1) {  // the FP64 part of a mixed build: the quartets on this kernel's side of SPLIT_CUT that stay in it
+        if ((bra.qf * ket.qf < float(SPLIT_CUT)) != DF) return;
+        const float bound = quartet_bound(A, bra, ket);
+        if (bound < A.skip_cut32 || bound < A.fp32_cut32) return;
+    }
     if constexpr (NP == 32) {
         // the lanes' partial sums scattered over the warp (81 elements: 82 additions per lane, 405 where every lane
         // gets every sum), then the contraction by all lanes: (pp|pp) of water in STO-3G 112 -> 68 us, four waters
@@ -437,22 +465,7 @@ __global__ void __launch_bounds__(128) fock_jk_group(const FockArgs A, const Nor
     } else if constexpr (!DF) {
         quartet_item_group<LA, LB, LC, LD, UHF, double, NP>(A, nt, rys, bra, ket, bi == ki, part, gmask);
     } else {
-        unsigned npass = 0;
-        double v[Q::NF];
-        {
-            df acc[Q::NF];
-            shell_quartet_df64<LA, LB, LC, LD>(bra, ket, A.primsdf, A.rysdf, A.prim_cut32, A.rys_compat != 0, acc,
-                                               A.counters ? &npass : nullptr, part, NP);
-#pragma unroll
-            for (int o = 1; o < NP; o <<= 1)
-#pragma unroll
-                for (int f = 0; f < Q::NF; ++f)
-                    acc[f] = df_add(acc[f], {__shfl_xor_sync(gmask, acc[f].h, o), __shfl_xor_sync(gmask, acc[f].l, o)});
-#pragma unroll
-            for (int f = 0; f < Q::NF; ++f) v[f] = df_to_f64(acc[f]);
-        }
-        if (part == 0) digest_jk<LA, LB, LC, LD, UHF, double>(A, bra, ket, bi == ki, v, nt);
-        if (A.counters) count_flush(A, npass);
+        quartet_item_group_df<LA, LB, LC, LD, UHF, NP>(A, nt, bra, ket, bi == ki, part, gmask);
     }
 }
 

@@ -26,6 +26,11 @@ cudaError_t launch_fock_fp64_part(int bc, int kc, bool uhf, const FockArgs& A64,
 // That part's quartets in pairs of floats as a kernel of their own.
 cudaError_t launch_fock_df64_part(int bc, int kc, bool uhf, const FockArgs& A, const NormTable& nt, int grid,
                                   cudaStream_t stream);
+// The whole FP64 part of one class of a mixed build on stream s: classes of up to 32 quartets per SM with a warp per
+// quartet (plus four lanes for those that run in FP32), the others as the two kernels above.
+cudaError_t launch_mixed_fp64(int bc, int kc, bool uhf, FockArgs A, const FockArgs& A32, const NormTable& nt,
+                              const double* rys64, const float* rys32, int nsm, int ctas64, int ctasdf, bool demotes,
+                              cudaStream_t s, int* launches);
 cudaError_t launch_schwarz(int pc, const ShellPair* pairs, const PrimPair* prims, int begin, int count,
                            const NormTable& nt, const double* rys, double* q_out, cudaStream_t stream);
 

@@ -68,4 +68,28 @@ cudaError_t launch_fock_fp64_part(int bc, int kc, bool uhf, const FockArgs& A64,
     }
 }
 
+cudaError_t launch_mixed_fp64(int bc, int kc, bool uhf, FockArgs A, const FockArgs& A32, const NormTable& nt,
+                              const double* rys64, const float* rys32, int nsm, int ctas64, int ctasdf, bool demotes,
+                              cudaStream_t s, int* launches) {
+    const long long few = (long long)nsm * 32;
+    // below eight times that many quartets in the part (known to the device only) four lanes per quartet fill the
+    // SMs better than one
+    A.df_group_max = 8 * few;
+    cudaError_t e = cudaSuccess;
+    if (A.nwork <= few) {
+        for (bool df : {false, true})
+            if (e == cudaSuccess) e = launch_fock_group(bc, kc, uhf, A, A.nwork, df, 32, nt, rys64, s);
+        *launches += 2;
+        A.only_demoted = 1;
+        if (e != cudaSuccess || !(demotes || A.counters)) return e;
+    }
+    e = launch_fock_fp64_part(bc, kc, uhf, A, A32, nt, rys64, rys32, nsm * ctas64, s);
+    ++*launches;
+    if (e == cudaSuccess && A.nwork > A.df_group_max) {
+        e = launch_fock_df64_part(bc, kc, uhf, A, nt, nsm * ctasdf, s);
+        ++*launches;
+    }
+    return e;
+}
+
 }  // namespace ugb

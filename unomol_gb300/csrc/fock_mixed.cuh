@@ -12,8 +12,9 @@ constexpr int FP64_PARTS = 4;
 // density reaches the FP32 cut; a quartet whose bound times the largest |P| of its own six blocks (the density
 // elements it is contracted with) is below that cut runs in FP32 here (with the FP32 part's arguments A32),
 // under the same per-quartet error bound as the FP32 part's own quartets.  Of the others, those below SPLIT_CUT
-// are left to fock_jk_df64_part and the rest (few, and the costliest of the build: one lane each would leave
-// most of the issue slots idle) run in FP64.
+// are left to fock_jk_df64_part unless the part is small, and the rest (few, and the costliest of the build: one
+// lane each would leave most of the issue slots idle) run in FP64; classes of few quartets in all leave both to
+// fock_jk_group, a warp per quartet (full-density build of a water in STO-3G 1.01 -> 0.27 ms, of five in 6-31G 2.44 -> 1.17 ms).
 template <int LA, int LB, int LC, int LD, bool UHF>
 __device__ __forceinline__ void fock_group_fp64_part(const FockArgs& A64, const FockArgs& A32, const NormTable& nt,
                                                      const double* __restrict__ rys64, const float* __restrict__ rys32,
@@ -34,8 +35,9 @@ __device__ __forceinline__ void fock_group_fp64_part(const FockArgs& A64, const 
         if (A64.counters && part == 0) count_demoted(A64);
         quartet_item_group<LA, LB, LC, LD, UHF, float, NP>(A32, nt, rys32, bra, ket, bi == ki, part, gmask);
     } else if (bra.qf * ket.qf < float(SPLIT_CUT)) {
-        return;  // fock_jk_df64_part
-    } else {
+        if (A64.only_demoted || *A64.dyn_total > A64.df_group_max) return;  // fock_jk_group, fock_jk_df64_part
+        quartet_item_group_df<LA, LB, LC, LD, UHF, NP>(A64, nt, bra, ket, bi == ki, part, gmask);
+    } else if (!A64.only_demoted) {
         quartet_item_group<LA, LB, LC, LD, UHF, double, NP>(A64, nt, rys64, bra, ket, bi == ki, part, gmask);
     }
 }
@@ -58,6 +60,7 @@ __global__ void __launch_bounds__(128) fock_jk_fp64_part(const FockArgs A64, con
 // ms for 256 molecules; all in FP64 10.0 and 68.9 ms).
 template <int LA, int LB, int LC, int LD, bool UHF>
 __global__ void __launch_bounds__(128, LA + LB + LC + LD <= 1 ? 8 : 1) fock_jk_df64_part(const FockArgs A, const NormTable nt) {
+    if (*A.dyn_total <= A.df_group_max) return;  // the group kernel's
     const long long total = *A.dyn_total, step = (long long)gridDim.x * blockDim.x;
     for (long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x; g - (threadIdx.x & 31) < total; g += step)
         df_item<LA, LB, LC, LD, UHF>(A, nt, g);
