@@ -69,3 +69,31 @@ def test_screened_fp64_build_matches_stored_integrals(gpu, system, n, basis):
     G = t.form_g(P)
     t.store_integrals(native.STORE_RHF)
     assert np.abs(G - t.form_g(P)).max() <= _bound(b, np.abs(P).max())
+
+
+@pytest.mark.gpu
+def test_two_root_regime_edge(gpu):
+    """The reference's two-root form starts above T = 15, where it departs from the exact one by 3.5e-4.  Two
+    centres at distances that put T of their (ps|ps) quartets within a few 2^-24 of 15 on both sides: the pairs
+    of floats and the FP64 integrals take the same side, whatever the parts of T."""
+    from unomol_gb300 import native
+    from unomol_gb300.basis import Basis
+    worst = 0.0
+    for a, c in ((0.5, 0.5), (0.37, 0.61), (0.83, 0.29)):
+        p, q = 2 * a, 2 * c  # both pairs on one centre each
+        for k in range(-12, 13):
+            R = np.sqrt(15.0 * (1.0 + (k + 0.5) * 2.0 ** -25) * (p + q) / (p * q))
+            d = np.array([0.36, 0.48, 0.8]) * R
+            text = "\n".join(["4 8 2 1", "2 50", "1e-10", "0 0", "2 1 0", "0 0 0", "1.0 0.0 0.0 0.0",
+                              f"1.0 {d[0]!r} {d[1]!r} {d[2]!r}"]
+                             + [f"1 {l} {x}\n{e!r} 1.0" for x, e in ((0, a), (1, c)) for l in (0, 1)]) + "\n"
+            text = text.replace("np.float64(", "").replace(")", "")
+            b = Basis(text=text)
+            P = rand_density(b.norb, 4)
+            t = native.TwoElectronInts(b)
+            t.set_precision(native.PREC_MIXED, 0.0)  # the screened FP64 build: its quartets in both forms
+            t.set_density_screening(0.0)
+            G = t.form_g(P)
+            t.store_integrals(native.STORE_RHF)
+            worst = max(worst, float(np.abs(G - t.form_g(P)).max()))
+    assert worst <= 1e-10

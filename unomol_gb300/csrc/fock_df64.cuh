@@ -55,6 +55,11 @@ __device__ __forceinline__ df df_poly(const float* __restrict__ c, float yh, flo
 // Interval k and local coordinate y = yh + yl = 2 (T / H - k) - 1 of T.  above: intervals (k H, (k + 1) H],
 // for the two-root tables (the reference's form starts above T = 15 and ends at T = 40); else [k H, (k + 1) H).
 __device__ __forceinline__ int df_index(bool above, df T, float& yh, float& yl) {
+    if (above) {  // the leading part as the rounded sum, so that it and the sign of the rest tell the side of 15
+        const float s = __fadd_rn(T.h, T.l);
+        T.l = __fsub_rn(T.l, __fsub_rn(s, T.h));
+        T.h = s;
+    }
     const float f = 4.0f * T.h;
     int k;
     if (above) {
