@@ -18,6 +18,12 @@ struct df {
 __device__ __forceinline__ df df_neg(df a) { return {-a.h, -a.l}; }
 __device__ __forceinline__ df df_half(df a) { return {__fmul_rn(0.5f, a.h), __fmul_rn(0.5f, a.l)}; }
 
+// the same sum with h its rounded value and l the exact rest (|a.h| >= |a.l|)
+__device__ __forceinline__ df df_norm(df a) {
+    const float s = __fadd_rn(a.h, a.l);
+    return {s, __fsub_rn(a.l, __fsub_rn(s, a.h))};
+}
+
 // a b
 __device__ __forceinline__ df df_mul(df a, df b) {
     const float p = __fmul_rn(a.h, b.h);
