@@ -22,3 +22,9 @@ def test_root_tables_are_read_inside_their_blocks(tmp_path):
     out = _run(tmp_path, "df_roots_main")
     looked, wrong = (int(v) for v in out.strip().split("\n")[-1].split())
     assert looked > 1_000_000 and wrong == 0, out
+
+
+def test_squares_of_differences(tmp_path):
+    """(P - Q)^2 of close product centres: nothing of the size of an ulp of the coordinates, squared, is lost."""
+    looked, wrong = (int(v) for v in _run(tmp_path, "df_diff_main").split())
+    assert looked == 320_000 and wrong == 0, wrong

@@ -53,6 +53,9 @@ __device__ __forceinline__ df df_add(df a, df b) {
     return {s, __fadd_rn(e, __fadd_rn(a.l, b.l))};
 }
 __device__ __forceinline__ df df_sub(df a, df b) { return df_add(a, df_neg(b)); }
+// a - b, normalised: of two close values what is left of l is up to half an ulp of a and not of the difference, and
+// the products, which leave out l l, would then be off by its square
+__device__ __forceinline__ df df_diff(df a, df b) { return df_norm(df_sub(a, b)); }
 // a b + c, any magnitudes
 __device__ __forceinline__ df df_fma(df a, df b, df c) { return df_add(c, df_mul(a, b)); }
 // f - a for |f| >= |a|

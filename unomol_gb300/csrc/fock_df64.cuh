@@ -133,7 +133,7 @@ __device__ __forceinline__ void shell_quartet_df64(const ShellPair& bra, const S
         const df rs = df_rsqrt(df_add(bp.p, kp.p));
         const df sr = df_mul(df_mul(bp.Ecc, kp.Ecc), rs);
         const df rpq = df_sqr(rs);
-        const df PQx = df_sub(bp.P[0], kp.P[0]), PQy = df_sub(bp.P[1], kp.P[1]), PQz = df_sub(bp.P[2], kp.P[2]);
+        const df PQx = df_diff(bp.P[0], kp.P[0]), PQy = df_diff(bp.P[1], kp.P[1]), PQz = df_diff(bp.P[2], kp.P[2]);
         const df R2 = df_add(df_add(df_sqr(PQx), df_sqr(PQy)), df_sqr(PQz));
         const df T = df_mul(df_mul(df_mul(bp.p, kp.p), rpq), R2);
         df x[NR], w[NR];
