@@ -27,7 +27,7 @@ def _tolerance(b, P):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("half,bits", [(8.0, 33), (512.0, 33)])
+@pytest.mark.parametrize("half,bits", [(8.0, 33), (512.0, 33), (262144.0, 33)])
 def test_two_fragments_far_apart(gpu, half, bits):
     from unomol_gb300 import native
     from unomol_gb300.basis import Basis

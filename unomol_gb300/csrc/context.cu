@@ -93,6 +93,7 @@ struct UnomolCtx {
     PrimPair* d_prims = nullptr;
     PrimPair32* d_prims32 = nullptr;
     PrimPairDF* d_primsdf = nullptr;
+    PairCentre* d_pcen = nullptr;
     BlockPair* d_bps = nullptr;
     long long* d_prefix = nullptr;
     double* d_rys = nullptr;
@@ -441,6 +442,7 @@ int build_setup(UnomolCtx* ctx) {
             ctx->d_prims = c.take<PrimPair>(nprims);
             ctx->d_prims32 = c.take<PrimPair32>(nprims);
             ctx->d_primsdf = c.take<PrimPairDF>(nprims);
+            ctx->d_pcen = c.take<PairCentre>(P);
         };
         Carve lay;
         recs(lay);
@@ -579,17 +581,10 @@ int build_setup(UnomolCtx* ctx) {
         CU(cudaMemcpyAsync(a.bbegin, ctx->block_begin.data(), sizeof(int) * nb, cudaMemcpyHostToDevice, s));
         CU(cudaMemcpyAsync(a.bcount, ctx->block_count.data(), sizeof(int) * nb, cudaMemcpyHostToDevice, s));
         CU(cudaMemcpyAsync(a.bprim, bprim.data(), sizeof(long long) * nb, cudaMemcpyHostToDevice, s));
-        double origin[3];  // the middle of the molecule's box
-        for (int k = 0; k < 3; ++k) {
-            double lo = ctx->centers[k], hi = lo;
-            for (int c = 1; c < ctx->ncen; ++c) {
-                lo = std::min(lo, ctx->centers[3 * c + k]);
-                hi = std::max(hi, ctx->centers[3 * c + k]);
-            }
-            origin[k] = 0.5 * (lo + hi);
-        }
-        CU(setup_interleave_prims(ctx->d_pairs, P, a.bbegin, a.bcount, a.bprim, nb, a.prims_c, a.prims32_c, ctx->d_prims,
-                                  ctx->d_prims32, ctx->d_primsdf, origin, s));
+        double far = 0.0;
+        for (double x : ctx->centers) far = std::max(far, std::fabs(x));
+        CU(setup_interleave_prims(sh, ctx->d_pairs, P, a.bbegin, a.bcount, a.bprim, nb, a.prims_c, a.prims32_c, ctx->d_prims,
+                                  ctx->d_prims32, ctx->d_primsdf, ctx->d_pcen, centre_step(far), s));
         CU(cudaStreamSynchronize(s));  // the host arrays above are copied from pageable memory
     }
     return build_worklists(ctx);
@@ -742,6 +737,7 @@ int fock_device(UnomolCtx* ctx, const double* dPa, const double* dPb, double* dG
     A.prims = ctx->d_prims;
     A.prims32 = ctx->d_prims32;
     A.primsdf = ctx->d_primsdf;
+    A.pcen = ctx->d_pcen;
     A.rysdf = ctx->d_rysdf;
     A.nbf = n;
     A.Pa = ctx->d_Pa;
@@ -967,6 +963,7 @@ CtxView ctx_view(const UnomolCtx* c) {
     v.d_prims = c->d_prims;
     v.d_prims32 = c->d_prims32;
     v.d_primsdf = c->d_primsdf;
+    v.d_pcen = c->d_pcen;
     v.nprims = c->nprims;
     v.d_prefix = c->d_prefix;
     v.d_bps = c->d_bps;
@@ -1462,6 +1459,7 @@ extern "C" int unomol_gpu_fock_rhf_noalloc(UnomolCtx* ctx, const double* dP, dou
     A.prims = ctx->d_prims;
     A.prims32 = ctx->d_prims32;
     A.primsdf = ctx->d_primsdf;
+    A.pcen = ctx->d_pcen;
     A.rysdf = ctx->d_rysdf;
     A.nbf = n;
     A.Pa = Pfull;

@@ -24,6 +24,7 @@ struct CtxView {
     const PrimPair* d_prims = nullptr;
     const PrimPair32* d_prims32 = nullptr;
     const PrimPairDF* d_primsdf = nullptr;
+    const PairCentre* d_pcen = nullptr;
     long long nprims = 0;
     const long long* d_prefix = nullptr;
     const BlockPair* d_bps = nullptr;  // device block pairs (the class launches' ranges index them)

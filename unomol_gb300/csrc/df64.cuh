@@ -53,6 +53,12 @@ __device__ __forceinline__ df df_add(df a, df b) {
     return {s, __fadd_rn(e, __fadd_rn(a.l, b.l))};
 }
 __device__ __forceinline__ df df_sub(df a, df b) { return df_add(a, df_neg(b)); }
+// a - c of two sums of three floats on common steps (PairCentre): the differences of the first and of the second parts
+// are exact, and the first is zero or at least as large as the second
+__device__ __forceinline__ df df_triple_diff(float ah, float am, float al, float ch, float cm, float cl) {
+    const float h = __fsub_rn(ah, ch), m = __fsub_rn(am, cm), s = __fadd_rn(h, m);
+    return {s, __fadd_rn(__fsub_rn(m, __fsub_rn(s, h)), __fsub_rn(al, cl))};
+}
 // a - b, normalised: of two close values what is left of l is up to half an ulp of a and not of the difference, and
 // the products, which leave out l l, would then be off by its square
 __device__ __forceinline__ df df_diff(df a, df b) { return df_norm(df_sub(a, b)); }

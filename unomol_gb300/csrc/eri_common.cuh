@@ -52,13 +52,19 @@ struct __align__(16) PrimPair32 {
     float pad_;     // 48 bytes: three 16-byte loads
 };
 
-// The record in pairs of floats (48 bits, df64.cuh), for the quartets below SPLIT_CUT.  P is taken relative
-// to the middle of the molecule's box: only differences of centres are used, and their rounding follows the
-// distance to the origin.
+// The record in pairs of floats (48 bits, df64.cuh), for the quartets below SPLIT_CUT.  It holds no product
+// centre: P - Q is A - C + (P - A) - (Q - C), whose rounding follows the distances inside the quartet and not
+// the molecule's extent.
 struct __align__(16) PrimPairDF {
     df p, E;        // first 16-byte load: the prefactor screen
     df Ecc, rp;
-    df P[3], PA[3];  // 80 bytes: five 16-byte loads
+    df PA[3];       // 64 bytes: four 16-byte loads
+};
+
+// Centre A of a shell pair as sums of three floats, per axis h + m + l: h a multiple of the molecule's centre
+// step, m of 2^-24 of it, so that differences of the first two are exact (setup.cu: centre_step).
+struct __align__(16) PairCentre {
+    float4 x, y, z;  // .w unused
 };
 
 // Schwarz bound from which a quartet of the FP64 build is evaluated in FP64; below it, in pairs of floats
@@ -114,6 +120,7 @@ struct FockArgs {
     const PrimPair* prims;
     const PrimPair32* prims32;
     const PrimPairDF* primsdf;
+    const PairCentre* pcen;
     const float* rysdf;         // root tables of the pairs-of-floats kernels
     const BlockPair* bps;
     const long long* prefix;    // concatenated staircase prefix sums

@@ -125,6 +125,7 @@ struct UnomolBatch {
     int nbps = 0;
     PrimPair32* d_prims32 = nullptr;
     PrimPairDF* d_primsdf = nullptr;
+    PairCentre* d_pcen = nullptr;
     // the FP64 build's split at SPLIT_CUT over the merged staircases (as one context's): one allocation
     char* d_split = nullptr;
     long long *d_pre_hi = nullptr, *d_pre_lo = nullptr, *d_cnt_hi = nullptr, *d_cnt_lo = nullptr;
@@ -187,6 +188,7 @@ FockArgs batch_args(UnomolBatch* b, const BLaunch& L, int k) {
     A.mode = 0;
     A.prims32 = b->d_prims32;
     A.primsdf = b->d_primsdf;
+    A.pcen = b->d_pcen;
     A.rysdf = b->rysdf;
     A.Pa32 = b->d_Pfull32;
     A.pmax = b->d_pmax;
@@ -550,6 +552,7 @@ int unomol_gpu_batch_create(const UnomolBasisDesc* bases, int nmol, UnomolBatch*
     BCU(cudaMalloc(&b->d_pairs, sizeof(ShellPair) * std::max<long long>(1, npair_tot)));
     BCU(cudaMalloc(&b->d_prims, sizeof(PrimPair) * std::max<long long>(1, nprim_tot)));
     BCU(cudaMalloc(&b->d_primsdf, sizeof(PrimPairDF) * std::max<long long>(1, nprim_tot)));
+    BCU(cudaMalloc(&b->d_pcen, sizeof(PairCentre) * std::max<long long>(1, npair_tot)));
     BCU(cudaMalloc(&b->d_bps, sizeof(BlockPair) * std::max<size_t>(1, bps.size())));
     BCU(cudaMalloc(&b->d_prefix, sizeof(long long) * std::max<long long>(1, nrow_tot)));
     // the molecules' device set-ups side by side: pairs point into the merged primitive array and carry
@@ -559,6 +562,7 @@ int unomol_gpu_batch_create(const UnomolBasisDesc* bases, int nmol, UnomolBatch*
         if (v.npairs > 0) {
             BCU(cudaMemcpyAsync(b->d_pairs + pair0s[m], v.d_pairs, sizeof(ShellPair) * v.npairs, cudaMemcpyDeviceToDevice, b->stream));
             BCU(setup_offset_pairs(b->d_pairs + pair0s[m], v.npairs, prim0s[m], m, b->stream));
+            BCU(cudaMemcpyAsync(b->d_pcen + pair0s[m], v.d_pcen, sizeof(PairCentre) * v.npairs, cudaMemcpyDeviceToDevice, b->stream));
         }
         if (v.nprims > 0)
             BCU(cudaMemcpyAsync(b->d_prims + prim0s[m], v.d_prims, sizeof(PrimPair) * v.nprims, cudaMemcpyDeviceToDevice, b->stream));
@@ -745,6 +749,7 @@ void unomol_gpu_batch_destroy(UnomolBatch* b) {
     dfree(b->d_T);
     dfree(b->d_prims32);
     dfree(b->d_primsdf);
+    dfree(b->d_pcen);
     dfree(b->d_split);
     dfree(b->d_Pfull32);
     dfree(b->d_pmax);

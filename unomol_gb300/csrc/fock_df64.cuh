@@ -105,10 +105,17 @@ __device__ __forceinline__ df pair_ab(const ShellPair& p, int k) {
     return {p.ABf[k], k == 0 ? p.ABl0 : k == 1 ? p.ABl1 : p.ABl2};
 }
 
+// A - C of a quartet's bra and ket
+__device__ __forceinline__ void centre_diff(const PairCentre& a, const PairCentre& c, df (&AC)[3]) {
+    AC[0] = df_triple_diff(a.x.x, a.x.y, a.x.z, c.x.x, c.x.y, c.x.z);
+    AC[1] = df_triple_diff(a.y.x, a.y.y, a.y.z, c.y.x, c.y.y, c.y.z);
+    AC[2] = df_triple_diff(a.z.x, a.z.y, a.z.z, c.z.x, c.z.y, c.z.z);
+}
+
 // Contracted integrals of one shell quartet as shell_quartet_eri<..., double>, in double-float: the same
 // primitive quartets (prefactor screen on floats, decided in double-float within 0.1 % of the cut).
 template <int LA, int LB, int LC, int LD>
-__device__ __forceinline__ void shell_quartet_df64(const ShellPair& bra, const ShellPair& ket,
+__device__ __forceinline__ void shell_quartet_df64(const ShellPair& bra, const ShellPair& ket, const df (&AC)[3],
                                                    const PrimPairDF* __restrict__ prims, const float* __restrict__ tab,
                                                    float prim_cut32, bool compat, df (&acc)[QClass<LA, LB, LC, LD>::NF],
                                                    unsigned* npass, int part = 0, int nparts = 1) {
@@ -128,12 +135,16 @@ __device__ __forceinline__ void shell_quartet_df64(const ShellPair& bra, const S
         if (v32 <= hi32 && !df_passes(bp_p, bp_E, kp_p, kp_E)) return false;
         return true;
     };
-    auto primitive = [&](const PrimPairDF& bp, const PrimPairDF& kp) {
+    // P - Q = AC + (P - A) - (Q - C), normalised before it is squared; AC with the record of the outer loop in `base`
+    auto with_bra = [&](const PrimPairDF& bp, df (&base)[3]) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) base[k] = df_add(AC[k], bp.PA[k]);
+    };
+    auto primitive = [&](const PrimPairDF& bp, const PrimPairDF& kp, const df& PQx, const df& PQy, const df& PQz) {
         if (npass) ++*npass;
         const df rs = df_rsqrt(df_add(bp.p, kp.p));
         const df sr = df_mul(df_mul(bp.Ecc, kp.Ecc), rs);
         const df rpq = df_sqr(rs);
-        const df PQx = df_diff(bp.P[0], kp.P[0]), PQy = df_diff(bp.P[1], kp.P[1]), PQz = df_diff(bp.P[2], kp.P[2]);
         const df R2 = df_add(df_add(df_sqr(PQx), df_sqr(PQy)), df_sqr(PQz));
         const df T = df_mul(df_mul(df_mul(bp.p, kp.p), rpq), R2);
         df x[NR], w[NR];
@@ -186,7 +197,10 @@ __device__ __forceinline__ void shell_quartet_df64(const ShellPair& bra, const S
             const int ib = t / nk, ik = t - ib * nk;
             const PrimPairDF bp = pb[ib * sb];
             const PrimPairDF kp = pk[ik * sk];
-            if (passes(bp.p, bp.E, kp.p, kp.E)) primitive(bp, kp);
+            if (!passes(bp.p, bp.E, kp.p, kp.E)) continue;
+            df base[3];
+            with_bra(bp, base);
+            primitive(bp, kp, df_diff(base[0], kp.PA[0]), df_diff(base[1], kp.PA[1]), df_diff(base[2], kp.PA[2]));
         }
         return;
     }
@@ -194,6 +208,8 @@ __device__ __forceinline__ void shell_quartet_df64(const ShellPair& bra, const S
         int ib = 0, ik = 0, cb = -1;
         float rowf = 0.f;  // bound of SRTERM E_ab / sqrt(p + q) over the kets
         PrimPairDF bp = pb[0];
+        df base[3];
+        with_bra(bp, base);
         for (;;) {
             PrimPairDF kp;
             bool found = false;
@@ -202,6 +218,7 @@ __device__ __forceinline__ void shell_quartet_df64(const ShellPair& bra, const S
                     bp = pb[ib * sb];
                     cb = ib;
                     rowf = float(SRTERM) * bp.E.h * rsqrtf(bp.p.h);
+                    with_bra(bp, base);
                 }
                 kp = pk[ik * sk];
                 if (rowf * kp.E.h < lo32) {  // E_cd descends: no later ket primitive passes either
@@ -218,17 +235,21 @@ __device__ __forceinline__ void shell_quartet_df64(const ShellPair& bra, const S
                 break;
             }
             if (!found) break;
-            primitive(bp, kp);
+            primitive(bp, kp, df_diff(base[0], kp.PA[0]), df_diff(base[1], kp.PA[1]), df_diff(base[2], kp.PA[2]));
         }
     } else {
         for (int ik = 0; ik < nk; ++ik) {
             const PrimPairDF kp = pk[ik * sk];
             const float colf = float(SRTERM) * kp.E.h * rsqrtf(kp.p.h);
+            df base[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) base[k] = df_sub(AC[k], kp.PA[k]);
             for (int ib = 0; ib < nb; ++ib) {
                 const PrimPairDF bp = pb[ib * sb];
                 if (colf * bp.E.h < lo32) break;  // E_ab descends: no later bra primitive passes either
                 if (!passes(bp.p, bp.E, kp.p, kp.E)) continue;
-                primitive(bp, kp);
+                primitive(bp, kp, df_norm(df_add(base[0], bp.PA[0])), df_norm(df_add(base[1], bp.PA[1])),
+                          df_norm(df_add(base[2], bp.PA[2])));
             }
         }
     }
@@ -250,8 +271,9 @@ __device__ __forceinline__ void df_item(const FockArgs& A, const NormTable& nt, 
     unsigned npass = 0;
     double v[Q::NF];
     {
-        df acc[Q::NF];
-        shell_quartet_df64<LA, LB, LC, LD>(bra, ket, A.primsdf, A.rysdf, A.prim_cut32, A.rys_compat != 0, acc,
+        df acc[Q::NF], AC[3];
+        centre_diff(A.pcen[bi], A.pcen[ki], AC);
+        shell_quartet_df64<LA, LB, LC, LD>(bra, ket, AC, A.primsdf, A.rysdf, A.prim_cut32, A.rys_compat != 0, acc,
                                            A.counters ? &npass : nullptr);
 #pragma unroll
         for (int f = 0; f < Q::NF; ++f) v[f] = df_to_f64(acc[f]);
@@ -316,13 +338,14 @@ __host__ __device__ constexpr int group_smem() {
 // quartet_item_group (fock_kernels.cuh) in pairs of floats.
 template <int LA, int LB, int LC, int LD, bool UHF, int NP>
 __device__ __forceinline__ void quartet_item_group_df(const FockArgs& A, const NormTable& nt, const ShellPair& bra,
-                                                      const ShellPair& ket, bool same_pair, int part, unsigned gmask) {
+                                                      const ShellPair& ket, int bi, int ki, int part, unsigned gmask) {
     using Q = QClass<LA, LB, LC, LD>;
     unsigned npass = 0;
     double v[Q::NF];
     {
-        df acc[Q::NF];
-        shell_quartet_df64<LA, LB, LC, LD>(bra, ket, A.primsdf, A.rysdf, A.prim_cut32, A.rys_compat != 0, acc,
+        df acc[Q::NF], AC[3];
+        centre_diff(A.pcen[bi], A.pcen[ki], AC);
+        shell_quartet_df64<LA, LB, LC, LD>(bra, ket, AC, A.primsdf, A.rysdf, A.prim_cut32, A.rys_compat != 0, acc,
                                            A.counters ? &npass : nullptr, part, NP);
 #pragma unroll
         for (int o = 1; o < NP; o <<= 1)
@@ -332,7 +355,7 @@ __device__ __forceinline__ void quartet_item_group_df(const FockArgs& A, const N
 #pragma unroll
         for (int f = 0; f < Q::NF; ++f) v[f] = df_to_f64(acc[f]);
     }
-    if (part == 0) digest_jk<LA, LB, LC, LD, UHF, double>(A, bra, ket, same_pair, v, nt);
+    if (part == 0) digest_jk<LA, LB, LC, LD, UHF, double>(A, bra, ket, bi == ki, v, nt);
     if (A.counters) count_flush(A, npass);
 }
 
@@ -365,10 +388,12 @@ __global__ void __launch_bounds__(128) fock_jk_group(const FockArgs A, const Nor
         double* V = smem + (threadIdx.x >> 5) * group_smem<LA, LB, LC, LD>();
         unsigned npass = 0;
         std::conditional_t<DF, df, double> acc[Q::NF];
-        if constexpr (DF)
-            shell_quartet_df64<LA, LB, LC, LD>(bra, ket, A.primsdf, A.rysdf, A.prim_cut32, A.rys_compat != 0, acc,
+        if constexpr (DF) {
+            df AC[3];
+            centre_diff(A.pcen[bi], A.pcen[ki], AC);
+            shell_quartet_df64<LA, LB, LC, LD>(bra, ket, AC, A.primsdf, A.rysdf, A.prim_cut32, A.rys_compat != 0, acc,
                                                A.counters ? &npass : nullptr, part, NP);
-        else
+        } else
             shell_quartet_eri<LA, LB, LC, LD, double, PrimPair>(bra, ket, A.prims, rys, A.prim_cut, A.prim_cut32, A.rys_compat != 0,
                                                                 acc, A.counters ? &npass : nullptr, part, NP);
         int first = 0, count = Q::NF;
@@ -391,7 +416,7 @@ __global__ void __launch_bounds__(128) fock_jk_group(const FockArgs A, const Nor
     } else if constexpr (!DF) {
         quartet_item_group<LA, LB, LC, LD, UHF, double, NP>(A, nt, rys, bra, ket, bi == ki, part, gmask);
     } else {
-        quartet_item_group_df<LA, LB, LC, LD, UHF, NP>(A, nt, bra, ket, bi == ki, part, gmask);
+        quartet_item_group_df<LA, LB, LC, LD, UHF, NP>(A, nt, bra, ket, bi, ki, part, gmask);
     }
 }
 

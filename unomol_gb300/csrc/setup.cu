@@ -4,6 +4,7 @@
 // builds its records, CUB radix sorts order them into blocks and, after the Schwarz diagonal, by
 // descending bound inside every block; one CTA per block pair binary-searches the Schwarz staircase of
 // its bra rows and a device scan turns the row counts into the prefix sums that the Fock kernels decode.
+#include <cmath>
 #include <cub/cub.cuh>
 
 #include "setup.h"
@@ -160,18 +161,23 @@ __device__ __forceinline__ df split_df(double v) {
     return {h, (float)(v - (double)h)};
 }
 
+__device__ __forceinline__ float4 split_centre(double v, double step) {
+    const double h = rint(v / step) * step, r = v - h, fine = step * 0x1p-24, m = rint(r / fine) * fine;
+    return make_float4((float)h, (float)m, (float)(r - m), 0.f);
+}
+
 // Final layout of the primitive pairs: block b (pairs bbegin[b] .. + bcount[b], all with the same
 // primitive-pair count) owns records bprim[b] .. + bcount[b] * nprim, and primitive ik of its j-th pair
 // sits at bprim[b] + ik * bcount[b] + j, so that the lanes of a warp, which hold consecutive pairs of a
 // block, read adjacent records.  src is the canonical layout, which dst32 keeps within a pair; dst has a
 // pair's records in descending E (equal ones in canonical order), which puts the primitive quartets past the prefactor screen first, at
-// the same places for the neighbouring pairs of a warp.  dstdf: the same records in pairs of floats, P
-// relative to `org`.  One warp per pair, each lane finding the rank of its records.
-__global__ void k_interleave_prims(ShellPair* __restrict__ pairs, int n, const int* __restrict__ bbegin,
+// the same places for the neighbouring pairs of a warp.  dstdf: the same records in pairs of floats; dstc:
+// the pairs' centres.  One warp per pair, each lane finding the rank of its records.
+__global__ void k_interleave_prims(const ShellsDev sh, ShellPair* __restrict__ pairs, int n, const int* __restrict__ bbegin,
                                    const int* __restrict__ bcount, const long long* __restrict__ bprim, int nb,
                                    const PrimPair* __restrict__ src, const PrimPair32* __restrict__ src32,
                                    PrimPair* __restrict__ dst, PrimPair32* __restrict__ dst32,
-                                   PrimPairDF* __restrict__ dstdf, double3 org) {
+                                   PrimPairDF* __restrict__ dstdf, PairCentre* __restrict__ dstc, double step) {
     const int k = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (k >= n) return;  // whole warps
     int lo = 0, hi = nb - 1;  // the block: last with bbegin <= k
@@ -199,14 +205,14 @@ __global__ void k_interleave_prims(ShellPair* __restrict__ pairs, int n, const i
         d.E = split_df(pp.E);
         d.Ecc = split_df(pp.Ecc);
         d.rp = split_df(pp.rp);
-        d.P[0] = split_df(pp.P[0] - org.x);
-        d.P[1] = split_df(pp.P[1] - org.y);
-        d.P[2] = split_df(pp.P[2] - org.z);
         for (int x = 0; x < 3; ++x) d.PA[x] = split_df(pp.PA[x]);
         dstdf[at] = d;
     }
     __syncwarp();
     if (lane == 0) {
+        const int ish = pairs[k].ish, jsh = pairs[k].jsh;
+        const double* A = sh.centers + 3 * sh.scen[sh.sl[ish] < sh.sl[jsh] ? jsh : ish];  // shell a, as k_build_pairs
+        dstc[k] = {split_centre(A[0], step), split_centre(A[1], step), split_centre(A[2], step)};
         pairs[k].prim_begin = (int)first;
         pairs[k].prim_stride = cnt;
     }
@@ -261,12 +267,19 @@ cudaError_t setup_row_bp(const BlockPair* bps, int nbp, int* row_bp, cudaStream_
     return cudaGetLastError();
 }
 
-cudaError_t setup_interleave_prims(ShellPair* pairs, int n, const int* bbegin, const int* bcount, const long long* bprim,
+// 2^-23 of the power of two at or above the largest |coordinate|: differences of multiples of it are floats
+double centre_step(double far) {
+    int e = 0;
+    std::frexp(std::fmax(far, 0x1p-20), &e);  // far < 2^e
+    return std::ldexp(1.0, e - 23);
+}
+
+cudaError_t setup_interleave_prims(const ShellsDev& sh, ShellPair* pairs, int n, const int* bbegin, const int* bcount, const long long* bprim,
                                    int nb, const PrimPair* src, const PrimPair32* src32, PrimPair* dst, PrimPair32* dst32,
-                                   PrimPairDF* dstdf, const double* origin, cudaStream_t s) {
+                                   PrimPairDF* dstdf, PairCentre* dstc, double step, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    k_interleave_prims<<<blocks_for(32ll * n, 128), 128, 0, s>>>(pairs, n, bbegin, bcount, bprim, nb, src, src32, dst, dst32,
-                                                         dstdf, make_double3(origin[0], origin[1], origin[2]));
+    k_interleave_prims<<<blocks_for(32ll * n, 128), 128, 0, s>>>(sh, pairs, n, bbegin, bcount, bprim, nb, src, src32, dst, dst32,
+                                                         dstdf, dstc, step);
     return cudaGetLastError();
 }
 

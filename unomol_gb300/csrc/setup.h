@@ -44,10 +44,11 @@ cudaError_t setup_row_bp(const BlockPair* bps, int nbp, int* row_bp, cudaStream_
 // primitive pairs of the sorted pairs moved from the canonical layout (src) into the block-interleaved
 // one (dst): block b's pairs bbegin[b] .. + bcount[b] own records bprim[b] .., primitive ik of its j-th
 // pair at bprim[b] + ik * bcount[b] + j; prim_begin / prim_stride of the pairs updated; dstdf: the records in
-// pairs of floats, P relative to origin (host, 3)
-cudaError_t setup_interleave_prims(ShellPair* pairs, int n, const int* bbegin, const int* bcount, const long long* bprim,
+// pairs of floats; dstc: the pairs' centres in steps of centre_step(largest |coordinate|)
+double centre_step(double far);
+cudaError_t setup_interleave_prims(const ShellsDev& sh, ShellPair* pairs, int n, const int* bbegin, const int* bcount, const long long* bprim,
                                    int nb, const PrimPair* src, const PrimPair32* src32, PrimPair* dst, PrimPair32* dst32,
-                                   PrimPairDF* dstdf, const double* origin, cudaStream_t s);
+                                   PrimPairDF* dstdf, PairCentre* dstc, double step, cudaStream_t s);
 // ShellPair::prim_begin += prim0 and ShellPair::pad = mol for n pairs (merging molecules into a batch)
 cudaError_t setup_offset_pairs(ShellPair* pairs, int n, int prim0, int mol, cudaStream_t s);
 
