@@ -28,3 +28,11 @@ def test_squares_of_differences(tmp_path):
     """(P - Q)^2 of close product centres: nothing of the size of an ulp of the coordinates, squared, is lost."""
     looked, wrong = (int(v) for v in _run(tmp_path, "df_diff_main").split())
     assert looked == 320_000 and wrong == 0, wrong
+
+
+def test_squares_have_no_bias(tmp_path):
+    """Rounding averages out over the quartets that a G element sums, a bias does not.  A value's error is about
+    2^-48 of it (32 units of 2^-53) at either sign, so the mean over 2 million values lies within 0.1 units of the bias.
+    The square of the low float, left out, is one of 6 units; an unnormalised reciprocal square root's, of 40."""
+    sq, rq = (float(v) for v in _run(tmp_path, "df_bias_main").split())
+    assert abs(sq) < 0.25 and abs(rq) < 4.0, (sq, rq)

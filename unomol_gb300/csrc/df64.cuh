@@ -32,11 +32,13 @@ __device__ __forceinline__ df df_mul(df a, df b) {
     e = __fmaf_rn(a.l, b.h, e);
     return {p, e};
 }
+// a^2.  l^2 counts although it lies below the last bit: it is never negative, so leaving it out, or adding it to a
+// value that is rounded already, would make every square too small, by 2^-50 of it on average, and sums over many
+// quartets keep such a bias where they average rounding away
 __device__ __forceinline__ df df_sqr(df a) {
     const float p = __fmul_rn(a.h, a.h);
-    float e = __fmaf_rn(a.h, a.h, -p);
-    e = __fmaf_rn(__fadd_rn(a.h, a.h), a.l, e);
-    return {p, e};
+    const float t = __fmaf_rn(__fadd_rn(a.h, a.h), a.l, __fmul_rn(a.l, a.l));
+    return {p, __fadd_rn(__fmaf_rn(a.h, a.h, -p), t)};
 }
 // a f with a single float f
 __device__ __forceinline__ df df_mulf(df a, float f) {
@@ -69,8 +71,8 @@ __device__ __forceinline__ df df_rsubf(float f, df a) {
     const float s = __fsub_rn(f, a.h);
     return {s, __fsub_rn(__fsub_rn(__fsub_rn(f, s), a.h), a.l)};
 }
-// 1 / sqrt(a), a > 0: the hardware approximation r and the series of (1 - e)^(-1/2) with e = 1 - a r^2 to
-// second order (|e| is about 2^-21, so what is left out is below 2^-60)
+// 1 / sqrt(a), a > 0, normalised (its square is taken): the hardware approximation r and the series of
+// (1 - e)^(-1/2) with e = 1 - a r^2 to second order (|e| is about 2^-21, so what is left out is below 2^-60)
 __device__ __forceinline__ df df_rsqrt(df a) {
     const float r = rsqrtf(a.h);
     const float q = __fmul_rn(r, r), ql = __fmaf_rn(r, r, -q);
@@ -80,7 +82,7 @@ __device__ __forceinline__ df df_rsqrt(df a) {
     t = __fmaf_rn(a.l, q, t);
     const float e = __fsub_rn(__fsub_rn(1.0f, p), t);
     const float c = __fmul_rn(__fmul_rn(r, e), __fmaf_rn(0.375f, e, 0.5f));
-    return {r, c};
+    return df_norm({r, c});
 }
 
 }  // namespace ugb
