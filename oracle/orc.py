@@ -73,6 +73,26 @@ def fock(b, Pa, Pb=None, exact=False, stride=1, offset=0, threads=0, start=0, ha
     return (Ga if Pb is None else (Ga, Gb)), cnt
 
 
+def fock_long(b, Ps, exact=False):
+    """[G(P)] (one density) or [Ga, Gb] in long double (np.longdouble), the inputs taken as they are: what the rounding
+    errors of a double-precision build are measured against."""
+    real = np.longdouble
+    L = C.CDLL(os.path.join(HERE, "_build", "libunomol_oracle_ld.so"))
+    L.orc_fock.argtypes = [C.c_void_p, C.c_int] + [C.c_void_p] * 4 + [C.c_int, C.c_longlong, C.c_longlong, C.c_int, C.c_void_p]
+    ints = [np.ascontiguousarray(v, np.int32) for v in (b.shell_l, b.shell_nprim, b.shell_center, b.shell_offset)]
+    reals = [np.ascontiguousarray(v, real).reshape(-1) for v in (b.alpha, b.coef, b.centers)]
+    d = _Basis(b.nshell, b.norb, b.ncen, *(k.ctypes.data_as(C.POINTER(C.c_int)) for k in ints),
+               *(C.cast(k.ctypes.data, C.POINTER(C.c_double)) for k in reals))  # the long double build's own pointers
+    P = [np.ascontiguousarray(p, real) for p in Ps]
+    G = [np.zeros(b.no2, real) for _ in P]
+    cnt = np.zeros(4, np.int64)
+    rc = L.orc_fock(C.addressof(d), 0, P[0].ctypes.data, P[1].ctypes.data if len(P) == 2 else None, G[0].ctypes.data,
+                    G[1].ctypes.data if len(P) == 2 else None, 1 if exact else 0, 1, 0, 0, cnt.ctypes.data)
+    if rc != 0:
+        raise RuntimeError(f"orc_fock failed ({rc})")
+    return G
+
+
 def records(b, exact=False, start=0):
     """The stored integrals of the reference's integral pass (TwoElectronInts.cpp:622-671): values and
     canonical labels (i, j, k, l) of every function quartet with |v| > 1e-14, in its loop order."""

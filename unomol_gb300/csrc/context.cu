@@ -600,7 +600,7 @@ __global__ void expand_packed(const double* __restrict__ pk, double* __restrict_
 }
 
 // G_packed[ij] += T[i][j] + T[j][i]
-__global__ void fold_packed(const double* __restrict__ T, double* __restrict__ G, int n) {
+__global__ void fold_packed(const double* __restrict__ T, double* __restrict__ G, int n, int copies) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long n2 = (long long)n * (n + 1) / 2;
     if (t >= n2) return;
@@ -609,21 +609,24 @@ __global__ void fold_packed(const double* __restrict__ T, double* __restrict__ G
     while ((long long)i * (i + 1) / 2 > t) --i;
     while ((long long)(i + 1) * (i + 2) / 2 <= t) ++i;
     const int j = (int)(t - (long long)i * (i + 1) / 2);
-    G[t] += T[(long long)i * n + j] + T[(long long)j * n + i];
+    double v = 0.0;
+    for (int c = 0; c < copies; ++c, T += (long long)n * n) v += T[(long long)i * n + j] + T[(long long)j * n + i];
+    G[t] += v;
 }
+
 
 int ensure_density_buffers(UnomolCtx* ctx, bool uhf) {
     const size_t n2 = (size_t)ctx->nbf * ctx->nbf;
     const size_t np = (size_t)ctx->nbf * (ctx->nbf + 1) / 2;
     if (!ctx->d_Pa) {
         CU(cudaMalloc(&ctx->d_Pa, n2 * sizeof(double)));
-        CU(cudaMalloc(&ctx->d_Ta, n2 * sizeof(double)));
+        CU(cudaMalloc(&ctx->d_Ta, acc_copies((long long)n2) * n2 * sizeof(double)));
         CU(cudaMalloc(&ctx->d_Ga, np * sizeof(double)));
         CU(cudaMalloc(&ctx->d_pk_a, np * sizeof(double)));
     }
     if (uhf && !ctx->d_Pb) {
         CU(cudaMalloc(&ctx->d_Pb, n2 * sizeof(double)));
-        CU(cudaMalloc(&ctx->d_Tb, n2 * sizeof(double)));
+        CU(cudaMalloc(&ctx->d_Tb, acc_copies((long long)n2) * n2 * sizeof(double)));
         CU(cudaMalloc(&ctx->d_Gb, np * sizeof(double)));
         CU(cudaMalloc(&ctx->d_pk_b, np * sizeof(double)));
     }
@@ -728,8 +731,9 @@ int fock_device(UnomolCtx* ctx, const double* dPa, const double* dPb, double* dG
         expand_packed<<<(unsigned)((n2 + 255) / 256), 256, 0, s>>>(dPb, ctx->d_Pb, n);
         ++launches;
     }
-    CU(cudaMemsetAsync(ctx->d_Ta, 0, n2 * sizeof(double), s));
-    if (uhf) CU(cudaMemsetAsync(ctx->d_Tb, 0, n2 * sizeof(double), s));
+    const int copies = acc_copies((long long)n2);
+    CU(cudaMemsetAsync(ctx->d_Ta, 0, copies * n2 * sizeof(double), s));
+    if (uhf) CU(cudaMemsetAsync(ctx->d_Tb, 0, copies * n2 * sizeof(double), s));
     CU(cudaGetLastError());
     CU(cudaEventRecord(ctx->ev[1], s));
     FockArgs A{};
@@ -744,6 +748,8 @@ int fock_device(UnomolCtx* ctx, const double* dPa, const double* dPb, double* dG
     A.Pb = uhf ? ctx->d_Pb : nullptr;
     A.Ta = ctx->d_Ta;
     A.Tb = uhf ? ctx->d_Tb : nullptr;
+    A.tmask = copies - 1;
+    A.tstride = (long long)n2;
     A.thr_int = STORE_CUT;
     A.prim_cut = PRIM_CUT;
     A.thr_int32 = (float)STORE_CUT;
@@ -857,10 +863,10 @@ int fock_device(UnomolCtx* ctx, const double* dPa, const double* dPb, double* dG
         }
     }
     CU(cudaEventRecord(ctx->ev[2], s));
-    fold_packed<<<(unsigned)((np + 255) / 256), 256, 0, s>>>(ctx->d_Ta, dGa, n);
+    fold_packed<<<(unsigned)((np + 255) / 256), 256, 0, s>>>(ctx->d_Ta, dGa, n, copies);
     ++launches;
     if (uhf) {
-        fold_packed<<<(unsigned)((np + 255) / 256), 256, 0, s>>>(ctx->d_Tb, dGb, n);
+        fold_packed<<<(unsigned)((np + 255) / 256), 256, 0, s>>>(ctx->d_Tb, dGb, n, copies);
         ++launches;
     }
     CU(cudaEventRecord(ctx->ev[3], s));
@@ -1452,7 +1458,8 @@ extern "C" int unomol_gpu_fock_rhf_noalloc(UnomolCtx* ctx, const double* dP, dou
     expand_packed<<<(unsigned)((n2 + 255) / 256), 256, 0, s>>>(dP, Pfull, n);
     ++launches;
     CU(cudaGetLastError());
-    CU(cudaMemsetAsync(T, 0, n2 * sizeof(double), s));  // the array keeps the previous call's sums
+    const int copies = acc_copies(n2, (long long)NOALLOC_SCRATCH_DOUBLES - n2);
+    CU(cudaMemsetAsync(T, 0, copies * n2 * sizeof(double), s));  // the array keeps the previous call's sums
     CU(cudaEventRecord(ctx->ev[1], s));
     FockArgs A{};
     A.pairs = ctx->d_pairs;
@@ -1466,6 +1473,8 @@ extern "C" int unomol_gpu_fock_rhf_noalloc(UnomolCtx* ctx, const double* dP, dou
     A.Pb = nullptr;
     A.Ta = T;
     A.Tb = nullptr;
+    A.tmask = copies - 1;
+    A.tstride = n2;
     A.thr_int = STORE_CUT;
     A.prim_cut = PRIM_CUT;
     A.thr_int32 = (float)STORE_CUT;
@@ -1476,7 +1485,7 @@ extern "C" int unomol_gpu_fock_rhf_noalloc(UnomolCtx* ctx, const double* dP, dou
     // the regular build's method selection: MD mode, runtime-L and MD classes included
     for (size_t li = 0; li < ctx->launches.size(); ++li) CU(launch_plain_class(ctx, li, false, A, s, s, launches));
     CU(cudaEventRecord(ctx->ev[2], s));
-    fold_packed<<<(unsigned)((np + 255) / 256), 256, 0, s>>>(T, dG, n);
+    fold_packed<<<(unsigned)((np + 255) / 256), 256, 0, s>>>(T, dG, n, copies);
     ++launches;
     CU(cudaEventRecord(ctx->ev[3], s));
     CU(cudaGetLastError());

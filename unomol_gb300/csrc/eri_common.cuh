@@ -114,6 +114,19 @@ struct BlockPair {
     long long work_count;       // quartets in this block pair
 };
 
+// Copies of the J/K accumulators that the CTAs share out; the fold adds them.  Why: each diagonal element of T takes one
+// addition per surviving ket pair (10^5 for 32 waters), each rounded at the running sum, and that, not the integrals, is
+// most of the error of G.  With c copies a copy takes 1/c of the additions at 1/c of the sum, and the errors add up to
+// 1/sqrt(c).  Against the oracle in long double (rms over G, 1e-15): 16 waters 8.2 with one copy, 3.8 with four, 3.4 with
+// eight (5.0 for one copy with the light classes first, when the large integrals come last); 32 waters 23.6, 7.6, 5.5
+// (10.4).  Fewer CTAs meet on an address, too: 32 waters 26.4 -> 23.9 ms.  Up to 1 GiB for all copies, then fewer.
+constexpr int ACC_COPIES = 8;
+inline int acc_copies(long long elements, long long room = 1ll << 27) {
+    int c = ACC_COPIES;
+    while (c > 1 && c * elements > room) c /= 2;
+    return c;
+}
+
 // Kernel arguments shared by every class instance.
 struct FockArgs {
     const ShellPair* pairs;
@@ -134,6 +147,8 @@ struct FockArgs {
     const float* pmax;          // shell-pair max |P| (nshell x nshell), for density screening
     double* Ta;                 // N x N accumulators; G = T + T^T
     double* Tb;                 // UHF beta accumulator
+    int tmask;                  // copies of the accumulators less one (acc_copies), tstride elements apart, taken
+    long long tstride;          // by the CTAs in turn
     double thr_int;             // per-integral cut (1e-14)
     double prim_cut;            // primitive prefactor cut (1e-12)
     float thr_int32, prim_cut32, skip_cut32;  // the same cuts in FP32, for the FP32 kernels

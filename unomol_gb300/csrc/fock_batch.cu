@@ -64,9 +64,10 @@ __global__ void batch_expand(const double* __restrict__ pk, const long long* __r
     full[t] = pk[poff[lo] + (long long)a * (a + 1) / 2 + b];
 }
 
-// packed G = T + T^T for every molecule
+// packed G = T + T^T, T the sum of the copies (stride elements apart), for every molecule
 __global__ void batch_fold(const double* __restrict__ T, const long long* __restrict__ doff, double* __restrict__ G,
-                           const long long* __restrict__ poff, const int* __restrict__ nbf, int nmol, long long total) {
+                           const long long* __restrict__ poff, const int* __restrict__ nbf, int nmol, long long total, int copies,
+                           long long stride) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= total) return;
     int lo = 0, hi = nmol - 1;
@@ -81,7 +82,9 @@ __global__ void batch_fold(const double* __restrict__ T, const long long* __rest
     while ((long long)(i + 1) * (i + 2) / 2 <= r) ++i;
     const int j = (int)(r - (long long)i * (i + 1) / 2);
     const double* Tm = T + doff[lo];
-    G[t] = Tm[(long long)i * n + j] + Tm[(long long)j * n + i];
+    double v = 0.0;
+    for (int c = 0; c < copies; ++c, Tm += stride) v += Tm[(long long)i * n + j] + Tm[(long long)j * n + i];
+    G[t] = v;
 }
 
 struct BLaunch {
@@ -177,6 +180,8 @@ FockArgs batch_args(UnomolBatch* b, const BLaunch& L, int k) {
     A.nbf = 0;
     A.Pa = b->d_Pfull;
     A.Ta = b->d_T;
+    A.tmask = acc_copies(b->dense_total) - 1;
+    A.tstride = b->dense_total;
     A.thr_int = STORE_CUT;
     A.prim_cut = PRIM_CUT;
     A.thr_int32 = (float)STORE_CUT;
@@ -236,7 +241,8 @@ int batch_build(UnomolBatch* b, cudaStream_t s) {
     batch_expand<<<(unsigned)((b->dense_total + 255) / 256), 256, 0, s>>>(b->d_P, b->d_poff, b->d_Pfull, b->d_doff, b->d_nbf,
                                                                           nmol, b->dense_total);
     BCU(cudaGetLastError());
-    BCU(cudaMemsetAsync(b->d_T, 0, sizeof(double) * b->dense_total, s));
+    const int copies = acc_copies(b->dense_total);
+    BCU(cudaMemsetAsync(b->d_T, 0, sizeof(double) * b->dense_total * copies, s));
     BCU(cudaMemsetAsync(b->d_tiles, 0, sizeof(unsigned long long) * 2 * std::max<size_t>(1, b->launches.size()), s));
     const bool mixed = b->prec_mode == UNOMOL_PREC_MIXED;
     if (mixed) {
@@ -300,7 +306,7 @@ int batch_build(UnomolBatch* b, cudaStream_t s) {
             BCU(cudaStreamWaitEvent(s, b->join[q], 0));
         }
     batch_fold<<<(unsigned)((b->packed_total + 255) / 256), 256, 0, s>>>(b->d_T, b->d_doff, b->d_G, b->d_poff, b->d_nbf,
-                                                                         nmol, b->packed_total);
+                                                                         nmol, b->packed_total, copies, b->dense_total);
     BCU(cudaGetLastError());
     return UNOMOL_OK;
 }
@@ -579,7 +585,7 @@ int unomol_gpu_batch_create(const UnomolBasisDesc* bases, int nmol, UnomolBatch*
     BCU(cudaMalloc(&b->d_P, sizeof(double) * packed));
     BCU(cudaMalloc(&b->d_G, sizeof(double) * packed));
     BCU(cudaMalloc(&b->d_Pfull, sizeof(double) * dense));
-    BCU(cudaMalloc(&b->d_T, sizeof(double) * dense));
+    BCU(cudaMalloc(&b->d_T, sizeof(double) * dense * acc_copies(dense)));
     BCU(cudaMalloc(&b->d_tiles, sizeof(unsigned long long) * 2 * std::max<size_t>(1, b->launches.size())));
     BCU(cudaMemcpy(b->d_bps, bps.data(), sizeof(BlockPair) * bps.size(), cudaMemcpyHostToDevice));
     b->nbps = (int)bps.size();
@@ -713,7 +719,7 @@ int unomol_gpu_batch_autotune(UnomolBatch* b, int reps, int* chosen) {
         cudaGraphExecDestroy(b->graph);
         b->graph = nullptr;
     }
-    BCU(cudaMemsetAsync(b->d_T, 0, sizeof(double) * b->dense_total, s));  // leave no partial sums
+    BCU(cudaMemsetAsync(b->d_T, 0, sizeof(double) * b->dense_total * acc_copies(b->dense_total), s));  // leave no partial sums
     BCU(cudaStreamSynchronize(s));
     return (int)b->launches.size();
 }

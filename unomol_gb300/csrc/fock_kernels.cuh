@@ -581,8 +581,9 @@ __device__ __forceinline__ void digest_jk(const FockArgs& A, const ShellPair& br
         N = A.mol_nbf[bra.pad];
         base = A.mol_base[bra.pad];
     }
-    double* __restrict__ Ta = A.Ta + base;
-    double* __restrict__ Tb = UHF ? A.Tb + base : nullptr;
+    const long long tcopy = base + (blockIdx.x & A.tmask) * A.tstride;
+    double* __restrict__ Ta = A.Ta + tcopy;
+    double* __restrict__ Tb = UHF ? A.Tb + tcopy : nullptr;
     // The degeneracy factor 1/2 per coincidence and the 4 (2) of the Coulomb sums are powers of two: applied
     // to the exponent fields, on the integer pipe (per (ss|ss) quartet 18 -> 7 FP64 instructions).
     const int ndeg = (bra.same() ? 1 : 0) + (ket.same() ? 1 : 0) + (same_pair ? 1 : 0);
@@ -707,6 +708,7 @@ __device__ __forceinline__ void digest_shared(const FockArgs& A, const ShellPair
         N = A.mol_nbf[bra.pad];
         off = A.mol_base[bra.pad];
     }
+    const long long toff = off + (blockIdx.x & A.tmask) * A.tstride;
     double* Pab = V + nab * vs;
     double* Pcd = Pab + nab;
     double* Pac = Pcd + ncd;
@@ -718,7 +720,7 @@ __device__ __forceinline__ void digest_shared(const FockArgs& A, const ShellPair
     const double jf = uhf ? 2.0 : 4.0;
     for (int spin = 0; spin < (uhf ? 2 : 1); ++spin) {
         const double* __restrict__ P = (spin ? A.Pb : A.Pa) + off;
-        double* __restrict__ T = (spin ? A.Tb : A.Ta) + off;
+        double* __restrict__ T = (spin ? A.Tb : A.Ta) + toff;
         auto block = [&](double* dst, int r0, int nrow, int col0, int ncol) {
             for (int e = lane; e < nrow * ncol; e += 32) dst[e] = __ldg(P + (long long)(r0 + e / ncol) * N + col0 + e % ncol);
         };
@@ -740,14 +742,14 @@ __device__ __forceinline__ void digest_shared(const FockArgs& A, const ShellPair
             for (int e = lane; e < nab; e += 32) {
                 double s = 0.0;
                 for (int k = 0; k < ncd; ++k) s = fma(V[e * vs + k], Pcd[k], s);
-                const long long o = off + (long long)(a0 + e / nb) * N + b0 + e % nb;
+                const long long o = toff + (long long)(a0 + e / nb) * N + b0 + e % nb;
                 atomicAdd(A.Ta + o, jf * s);
                 if (uhf) atomicAdd(A.Tb + o, jf * s);
             }
             for (int e = lane; e < ncd; e += 32) {
                 double s = 0.0;
                 for (int k = 0; k < nab; ++k) s = fma(V[k * vs + e], Pab[k], s);
-                const long long o = off + (long long)(c0 + e / nd) * N + d0 + e % nd;
+                const long long o = toff + (long long)(c0 + e / nd) * N + d0 + e % nd;
                 atomicAdd(A.Ta + o, jf * s);
                 if (uhf) atomicAdd(A.Tb + o, jf * s);
             }
