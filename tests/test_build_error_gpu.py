@@ -37,6 +37,7 @@ def error(b, P):
 @pytest.mark.gpu
 @pytest.mark.parametrize("system,n,basis,seed,density,most", [
     ("alkane", 7, "STO-3G", 3, "random", 2.24), ("alkane", 7, "STO-3G", 5, "random", 2.39),
+    ("alkane", 4, "6-31G", 3, "core", 2.38), ("water", 5, "6-31G", 3, "core", 2.31),
 ])
 def test_rounding_error_of_a_build(gpu, system, n, basis, seed, density, most):
     from unomol_gb300 import molecules

@@ -610,7 +610,11 @@ __global__ void fold_packed(const double* __restrict__ T, double* __restrict__ G
     while ((long long)(i + 1) * (i + 2) / 2 <= t) ++i;
     const int j = (int)(t - (long long)i * (i + 1) / 2);
     double v = 0.0;
-    for (int c = 0; c < copies; ++c, T += (long long)n * n) v += T[(long long)i * n + j] + T[(long long)j * n + i];
+    T += (long long)i * n + j;
+    const long long tr = (long long)(j - i) * (n - 1), step = (long long)n * n;  // tr: to element (j, i)
+#pragma unroll
+    for (int c = 0; c < ACC_COPIES; ++c)  // (unrolled: all loads in flight)
+        if (c < copies) v += T[c * step] + T[c * step + tr];
     G[t] += v;
 }
 
@@ -775,6 +779,7 @@ int fock_device(UnomolCtx* ctx, const double* dPa, const double* dPb, double* dG
         CU(wl_scan_launches(ctx->d_launch_bp, (int)ctx->launches.size(), ctx->d_cnt64, ctx->d_cnt32, ctx->d_begin64,
                             ctx->d_begin32, ctx->d_total64, ctx->d_total32, s));
         launches += 4;
+        A.split_cut32 = (float)(ctx->fp32_cut > ctx->skip_cut ? MIXED_SPLIT_CUT : SPLIT_CUT);
         A.dmax = ctx->d_dmax;
         A.skip_cut = ctx->skip_cut;
         A.skip_cut32 = (float)ctx->skip_cut;

@@ -68,11 +68,15 @@ struct __align__(16) PairCentre {
 };
 
 // Schwarz bound from which a quartet of the FP64 build is evaluated in FP64; below it, in pairs of floats
-// (fock_df64.cuh), whose error of about 2^-46 of the bound is then below 2e-15.  Chosen by the error of G
-// against the reference's fixtures, which stays what the all-FP64 build has up to a cut of 1/2 (a cut of 100,
-// every quartet in pairs of floats, doubles it on the three-water one), and by time (32 waters / n-decane
-// UHF): 1/128 24.7 / 5.3 ms, 1/32 23.2 / 4.6, 1/8 21.8 / 3.5, 1/2 20.4 / 3.4, 100 20.0 / 3.3.
-constexpr double SPLIT_CUT = 0.125;
+// (fock_df64.cuh), whose integrals are off by about 2^-50 of the bound (rms; s and p shells).  Chosen as the largest
+// for which the error of G stays what the all-FP64 build had with one accumulator per element.  Error of G against the
+// oracle in long double (rms, 1e-15; that build / a cut of 1/16 / of 1/8), densities of the core Hamiltonian: 6-31G
+// ethane 1.00 / 1.23 / 2.76, n-butane 2.38 / 2.14 / 4.64, five waters 2.31 / 1.89 / 2.50; STO-3G n-heptane
+// 3.09 / 2.90 / 5.44.  Time, 32 waters / n-decane UHF: 1/32 25.4 / 3.7 ms, 1/16 25.1 / 3.1, 1/8 23.9 / 2.7.
+// Builds with an FP32 part, whose error the caller sets, split their FP64 part at MIXED_SPLIT_CUT (32 waters, full
+// density: 9.45 ms at 1/16, 8.84 at 1/8).
+constexpr double SPLIT_CUT = 0.0625;
+constexpr double MIXED_SPLIT_CUT = 0.125;
 
 constexpr double SQRT_SRTERM = 5.914967172795613;  // sqrt(2 pi^{5/2})
 static_assert(SQRT_SRTERM * SQRT_SRTERM - SRTERM < 1e-13 && SRTERM - SQRT_SRTERM * SQRT_SRTERM < 1e-13, "sqrt of SRTERM");
@@ -152,6 +156,7 @@ struct FockArgs {
     double thr_int;             // per-integral cut (1e-14)
     double prim_cut;            // primitive prefactor cut (1e-12)
     float thr_int32, prim_cut32, skip_cut32;  // the same cuts in FP32, for the FP32 kernels
+    float split_cut32;          // FP64 part of a screened build: quartets with a Schwarz bound below this in pairs of floats
     int only_demoted;           // FP64 part of a mixed build: only its FP32 quartets (the others have a launch of their own)
     long long df_group_max;     // and up to this many quartets in the part it also takes the pairs-of-floats ones
     float fp32_cut32;           // mixed mode: a quartet with bound * max|P| of its blocks below this runs in FP32

@@ -83,7 +83,10 @@ __global__ void batch_fold(const double* __restrict__ T, const long long* __rest
     const int j = (int)(r - (long long)i * (i + 1) / 2);
     const double* Tm = T + doff[lo];
     double v = 0.0;
-    for (int c = 0; c < copies; ++c, Tm += stride) v += Tm[(long long)i * n + j] + Tm[(long long)j * n + i];
+    const long long ij = (long long)i * n + j, ji = (long long)j * n + i;
+#pragma unroll
+    for (int c = 0; c < ACC_COPIES; ++c)
+        if (c < copies) v += Tm[c * stride + ij] + Tm[c * stride + ji];
     G[t] = v;
 }
 
@@ -202,6 +205,7 @@ FockArgs batch_args(UnomolBatch* b, const BLaunch& L, int k) {
     A.skip_cut32 = (float)b->skip_cut;
     A.fp32_cut = b->fp32_cut;
     A.fp32_cut32 = b->fp32_cut > b->skip_cut ? (float)b->fp32_cut : 0.f;  // per-quartet FP32 choice of the FP64 part
+    A.split_cut32 = (float)(b->fp32_cut > b->skip_cut ? MIXED_SPLIT_CUT : SPLIT_CUT);
     A.dyn_mseg = b->d_mseg;
     A.mol_nshell = b->d_nshell;
     A.mol_pmax = b->d_pmax_off;

@@ -1,9 +1,8 @@
 // Shell-quartet integrals in pairs of floats (df64.cuh), for the quartets of the FP64 build whose Schwarz
-// bound lies below SPLIT_CUT.  The integrals of such a quartet are at most SPLIT_CUT, so the form's 2^-47
-// or so of the bound stays below half an ulp of an integral of order one, which every FP64 evaluation of
-// the larger quartets carries as well; the sum over the quartets, and with it G, keeps its error.  The
-// quartets above the cut are evaluated in FP64, and the density contraction and the accumulation are FP64
-// for all of them.
+// bound lies below SPLIT_CUT (1/16).  Their integrals come out within about 2^-50 of the bound (rms, s and p
+// shells), that is 2^-54, less than an FP64 evaluation of the quartets of order one is off; G keeps its error
+// (SPLIT_CUT's comment has the figures).  The quartets above the cut are evaluated in FP64, and the density
+// contraction and the accumulation are FP64 for all of them.
 //
 // What bounds it: the FP64 kernels keep the FP64 pipe (2 lanes per clock and SM) 88 % busy; the same
 // primitive quartet of (ps|ss) is about 65 FP64 instructions (1040 SM clocks per warp) or about 350 FP32
@@ -143,18 +142,20 @@ __device__ __forceinline__ void shell_quartet_df64(const ShellPair& bra, const S
     auto primitive = [&](const PrimPairDF& bp, const PrimPairDF& kp, const df& PQx, const df& PQy, const df& PQz) {
         if (npass) ++*npass;
         const df rs = df_rsqrt(df_add(bp.p, kp.p));
-        const df sr = df_mul(df_mul(bp.Ecc, kp.Ecc), rs);
-        const df rpq = df_sqr(rs);
-        const df R2 = df_add(df_add(df_sqr(PQx), df_sqr(PQy)), df_sqr(PQz));
-        const df T = df_mul(df_mul(df_mul(bp.p, kp.p), rpq), R2);
+        // the factors that the rest is made of are normalised: the error of an integral falls from 15 to 11 (ss|ss), 12
+        // to 7 (ps|ss) and 11 to 6 (ps|ps) units of 2^-53 of the bound (rms over random primitives)
+        const df sr = df_muln(df_muln(bp.Ecc, kp.Ecc), rs);
+        const df rpq = df_norm(df_sqr(rs));
+        const df R2 = df_norm(df_add(df_add(df_sqr(PQx), df_sqr(PQy)), df_sqr(PQz)));
+        const df T = df_mul(df_muln(df_muln(bp.p, kp.p), rpq), R2);
         df x[NR], w[NR];
         df_roots<NR, L12 + L34 != 0>(T, tab, compat, x, w);
         if constexpr (L12 + L34 == 0) {
-            acc[0] = df_fma(w[0], sr, acc[0]);
+            acc[0] = df_fma(df_norm(w[0]), sr, acc[0]);
         } else {
 #pragma unroll
             for (int r = 0; r < NR; ++r) {
-                const df fff = df_mul(x[r], rpq);  // t^2 / (p + q)   (Rys.hpp:126-129)
+                const df fff = df_muln(df_norm(x[r]), rpq);  // t^2 / (p + q)   (Rys.hpp:126-129)
                 const df zero = {0.f, 0.f};
                 const df qf = L12 > 0 ? df_mul(kp.p, fff) : zero, pf = L34 > 0 ? df_mul(bp.p, fff) : zero;
                 const df B00 = (L12 > 0 && L34 > 0) ? df_half(fff) : zero;
@@ -164,13 +165,14 @@ __device__ __forceinline__ void shell_quartet_df64(const ShellPair& bra, const S
                 df Ix[Q::NI], Iy[Q::NI], Iz[Q::NI];
                 const df nqf = df_neg(qf);
                 auto axis = [&](int k, const df& PQ, auto unit, df g, df(&I)[Q::NI]) {
-                    const df C = L12 > 0 ? df_fma(nqf, PQ, bp.PA[k]) : zero, Cp = L34 > 0 ? df_fma(pf, PQ, kp.PA[k]) : zero;
+                    const df C = L12 > 0 ? df_norm(df_fma(nqf, PQ, bp.PA[k])) : zero;
+                    const df Cp = L34 > 0 ? df_norm(df_fma(pf, PQ, kp.PA[k])) : zero;
                     const df AB = LB > 0 ? pair_ab(bra, k) : zero, CD = LD > 0 ? pair_ab(ket, k) : zero;
                     df_axis<LA, LB, LC, LD, decltype(unit)::value>(g, C, Cp, B00, B1, B1p, AB, CD, I);
                 };
                 axis(0, PQx, std::true_type{}, df{1.f, 0.f}, Ix);
                 axis(1, PQy, std::true_type{}, df{1.f, 0.f}, Iy);
-                axis(2, PQz, std::false_type{}, df_mul(w[r], sr), Iz);
+                axis(2, PQz, std::false_type{}, df_muln(df_norm(w[r]), sr), Iz);
 #pragma unroll
                 for (int ia = 0; ia < Q::NA; ++ia)
 #pragma unroll
@@ -264,7 +266,7 @@ __device__ __forceinline__ void df_item(const FockArgs& A, const NormTable& nt, 
     const ShellPair bra = A.pairs[bi];
     const ShellPair ket = A.pairs[ki];
     if (A.mode == 1) {  // the FP64 part of a mixed build: the others are the group kernel's
-        if (!(bra.qf * ket.qf < float(SPLIT_CUT))) return;
+        if (!(bra.qf * ket.qf < A.split_cut32)) return;
         const float bound = quartet_bound(A, bra, ket);
         if (bound < A.skip_cut32 || bound < A.fp32_cut32) return;
     }
@@ -375,7 +377,7 @@ __global__ void __launch_bounds__(128) fock_jk_group(const FockArgs A, const Nor
     const ShellPair bra = A.pairs[bi];
     const ShellPair ket = A.pairs[ki];
     if (A.mode == 1) {  // the FP64 part of a mixed build: the quartets on this kernel's side of SPLIT_CUT that stay in it
-        if ((bra.qf * ket.qf < float(SPLIT_CUT)) != DF) return;
+        if ((bra.qf * ket.qf < A.split_cut32) != DF) return;
         const float bound = quartet_bound(A, bra, ket);
         if (bound < A.skip_cut32 || bound < A.fp32_cut32) return;
     }

@@ -34,7 +34,7 @@ __device__ __forceinline__ void fock_group_fp64_part(const FockArgs& A64, const 
     if (bound < A64.fp32_cut32) {
         if (A64.counters && part == 0) count_demoted(A64);
         quartet_item_group<LA, LB, LC, LD, UHF, float, NP>(A32, nt, rys32, bra, ket, bi == ki, part, gmask);
-    } else if (bra.qf * ket.qf < float(SPLIT_CUT)) {
+    } else if (bra.qf * ket.qf < A64.split_cut32) {
         if (A64.only_demoted || *A64.dyn_total > A64.df_group_max) return;  // fock_jk_group, fock_jk_df64_part
         quartet_item_group_df<LA, LB, LC, LD, UHF, NP>(A64, nt, bra, ket, bi, ki, part, gmask);
     } else if (!A64.only_demoted) {
