@@ -50,9 +50,10 @@ __device__ __forceinline__ double f32_to_f64(float f) {
     const unsigned lo = e ? (u << 29) : 0u;
     return __hiloint2double((int)hi, (int)lo);
 }
-// v 2^n for a normal v whose result stays normal (the integrals past the storage cut)
+// v 2^n for a normal v whose result stays normal (the integrals past the storage cut); infinities and NaN stay
 __device__ __forceinline__ double scale_pow2(double v, int n) {
-    return __hiloint2double(__double2hiint(v) + n * (1 << 20), __double2loint(v));
+    const int hi = __double2hiint(v);
+    return __hiloint2double((~hi & 0x7ff00000) ? hi + n * (1 << 20) : hi, __double2loint(v));
 }
 __device__ __forceinline__ float scale_pow2(float v, int n) { return __int_as_float(__float_as_int(v) + n * (1 << 23)); }
 // v 2^n, n >= 0, for any v (zero, subnormal, infinite and NaN values by a product)
