@@ -85,7 +85,8 @@ template <int KF>
 __global__ void __launch_bounds__(32 * COOP_WARPS) fock_jk_coop(const FockArgs A, const NormTable nt, const double* __restrict__ rys,
                                                                 int la, int lb, int lc, int ld) {
     extern __shared__ double smem[];
-    if (A.mode != 0 && (long long)blockIdx.x * COOP_WARPS >= *A.dyn_total) return;  // past a screened list's end
+    const long long cta = (long long)blockIdx.y * gridDim.x + blockIdx.x;
+    if (A.mode != 0 && cta * COOP_WARPS >= *A.dyn_total) return;  // past a screened list's end
     const CoopShape q(la, lb, lc, ld);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     // CTA tables: per function quartet its element of the three axes, per transfer element (a, b, c, d), norms
@@ -107,7 +108,7 @@ __global__ void __launch_bounds__(32 * COOP_WARPS) fock_jk_coop(const FockArgs A
     for (int e = threadIdx.x; e < q.nab; e += blockDim.x) nab[e] = nt.v[la][e / q.nb] * nt.v[lb][e % q.nb];
     for (int e = threadIdx.x; e < q.ncd; e += blockDim.x) ncd[e] = nt.v[lc][e / q.nd] * nt.v[ld][e % q.nd];
     __syncthreads();
-    const long long w = (long long)blockIdx.x * COOP_WARPS + wid;
+    const long long w = cta * COOP_WARPS + wid;
     int bi, ki;
     if (!(A.mode == 0 ? decode_warp_items<false>(A, w, 0, bi, ki) : decode_warp_items<true>(A, w, 0, bi, ki))) return;
     const ShellPair bra = A.pairs[bi];
