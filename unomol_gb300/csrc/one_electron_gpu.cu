@@ -542,7 +542,9 @@ int one_electron_impl(const UnomolBasisDesc* b, const double* charges, int ngeom
                     return UNOMOL_EINVAL;
                 }
                 pairs[la + lb].push_back(la >= lb ? make_int2(sa, sb) : make_int2(sb, sa));
-                covered += sa == sb ? na * (na + 1) / 2 : na * nb;
+                for (int ca = 0; ca < na; ++ca)  // the elements (i, j), j <= i, as below: shells that overlap or come
+                    for (int cb = 0; cb < nb; ++cb)  // out of order are refused by their count
+                        covered += b->shell_offset[sb] + cb <= b->shell_offset[sa] + ca;
                 continue;
             }
             for (int ca = 0; ca < na; ++ca)
