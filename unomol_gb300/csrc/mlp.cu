@@ -298,7 +298,11 @@ int Mlp::forward(const float* x, int ldx, int r, cudaStream_t s) {
     if (rc) return rc;
     if (r > 0) k_to_bf16_pad<<<nblk((long long)r * n_in_pad), 256, 0, s>>>(x, ldx, r, n_in, n_in_pad, X);
     MLP_CK(cudaGetLastError());
-    return forward_x(r, s);
+    // a forward pass after one without a backward pass is taken for inference and writes no transposed activations (200000
+    // rows 1454 -> 1380 us); a backward pass that follows all the same makes them itself
+    const bool train = expect_backward;
+    expect_backward = false;
+    return forward_x(r, s, train);
 }
 
 int Mlp::forward_x(int r, cudaStream_t s, bool train) {
@@ -342,6 +346,7 @@ int Mlp::backward(const float* dy, bool accumulate, cudaStream_t s) {
         return UNOMOL_EINVAL;
     }
     if (!accumulate) MLP_CK(cudaMemsetAsync(G, 0, np_pad * sizeof(float), s));
+    expect_backward = true;
     const int r = rows;
     if (r == 0) return UNOMOL_OK;
     const int L = layers;

@@ -35,6 +35,7 @@ struct Mlp {
     __nv_bfloat16* dZb[2] = {nullptr, nullptr};  // [cap x hidden]
     std::vector<__nv_bfloat16*> HT;            // [layers][hidden x rows rounded up to 8]: H transposed, for the weight gradients
     bool have_t = false;                       // HT belongs to the last forward
+    bool expect_backward = true;               // forward(): a backward followed the one before (or there was none)
     __nv_bfloat16 *Ta = nullptr, *Tb = nullptr;  // transposed operands of the weight gradients
     int* status = nullptr;                     // device flag: a GEMM wait gave up
     std::string err;
