@@ -323,7 +323,8 @@ typedef struct UnomolScfOptions {
     double diis_start;   /* DIIS: extrapolate once the error is below this (<= 0: from the start) */
     double level_shift;  /* DIIS: virtual-orbital shift sigma (0: none) ... */
     double level_shift_until; /* ... applied while the DIIS error is above this */
-    int incremental;     /* 1: G(P) = G(P_prev) + G(P - P_prev) between full builds (new) */
+    int incremental;     /* 1: G(P) = G(P_prev) + G(P - P_prev) between full builds (new); in the precision
+                            form with a density-screening cut of at most 1e-3 eps */
     int rebuild_every;   /* incremental: a full build every this many builds (<= 0: 8) */
     int loop;            /* UNOMOL_SCF_LOOP_GROUND: the loop of findEnergy (two updates, then the
                             convergence test; RHF.hpp:138-162); UNOMOL_SCF_LOOP_DPM: the loop of

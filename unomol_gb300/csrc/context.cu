@@ -994,6 +994,8 @@ CtxView ctx_view(const UnomolCtx* c) {
     return v;
 }
 
+double ctx_skip_cut(const UnomolCtx* c) { return c->skip_cut; }
+
 }  // namespace ugb
 
 namespace {

@@ -44,5 +44,7 @@ struct CtxView {
 };
 
 CtxView ctx_view(const UnomolCtx* ctx);
+// skip_cut of the density-screened build
+double ctx_skip_cut(const UnomolCtx* ctx);
 
 }  // namespace ugb
