@@ -113,12 +113,17 @@ int unomol_gpu_fock_uhf_device(UnomolCtx* ctx, const double* dPa, const double* 
                                double* dGb, void* stream);
 
 /* Precision form (no reference counterpart; the reference is FP64 only).
- * UNOMOL_PREC_FP64 (default): every quartet that passes the integral Schwarz cut, in FP64.
+ * UNOMOL_PREC_FP64 (default): every quartet that passes the integral Schwarz cut.  Quartets whose Schwarz
+ *   bound sqrt((ab|ab)) sqrt((cd|cd)) is 1/16 or more are evaluated in FP64; those of s, p and d shells (up
+ *   to 81 function quartets) below it have their integrals evaluated in unevaluated sums of two floats (48
+ *   bits; off by about 2^-50 of the bound, 2^-54 in absolute terms, for s and p shells).  The density
+ *   contraction and all sums are FP64.  The error of G is that of a build with every quartet in FP64.
  * UNOMOL_PREC_MIXED: density-screened build made per call on the device.  With b = sqrt((ab|ab))
  *   sqrt((cd|cd)) and D = max |P| over the density passed in: quartets with b*D >= fp32_cutoff run in
- *   FP64, quartets with skip_cut <= b*D < fp32_cutoff in FP32 (Rys roots, recurrences, contraction and
- *   the density contraction of each quartet in FP32; its J/K sums added into G in FP64), the rest (and
- *   quartets whose six density blocks are all small) are skipped.  Meant for incremental builds
+ *   FP64 (as above; where there is an FP32 part, pairs of floats below a bound of 1/8), quartets with
+ *   skip_cut <= b*D < fp32_cutoff in FP32 (Rys roots, recurrences, contraction and the density contraction
+ *   of each quartet in FP32; its J/K sums added into G in FP64), the rest (and quartets whose six density
+ *   blocks are all small) are skipped.  Meant for incremental builds
  *   G(P) = G(P_old) + G(dP),
  *   where |dP| shrinks as the SCF converges.  fp32_cutoff <= skip_cut gives a density-screened FP64
  *   build. */
@@ -160,7 +165,8 @@ int unomol_gpu_get_stats(const UnomolCtx* ctx, UnomolStats* out);
 int unomol_gpu_set_counting(UnomolCtx* ctx, int on);
 
 /* Order of the class launches of a Fock build (no reference counterpart; a diagnostic control):
- * 0 (default) in class order, non-zero in reverse.  The J/K contributions meet in FP64 atomics, so the
+ * 0 (default): FP64 builds with the heaviest angular classes first, screened builds with the lightest first;
+ * non-zero: the other way round.  The J/K contributions meet in FP64 atomics, so the
  * order of the additions, and with it the rounding of G, changes from launch order to launch order and
  * from run to run; the determinism tests bound that difference. */
 int unomol_gpu_set_launch_order(UnomolCtx* ctx, int reversed);
