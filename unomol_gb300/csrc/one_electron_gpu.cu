@@ -424,13 +424,12 @@ __global__ void __launch_bounds__(128) k_one_sp(const OneArgs a, const int2* __r
         }
 }
 
-constexpr long long ONE_FEW = 152 * 64;
 template <int LA, int LB>
-void launch_sp(const OneArgs& a, const int2* pairs, int n, int ngeom) {
+void launch_sp(const OneArgs& a, const int2* pairs, int n, int ngeom, int nsm) {
     if (n <= 0) return;
     // four lanes per pair once that gives every SM two warps (16 n-decane geometries 3.15 ms; from eight warps on
     // 3.39), a warp per pair below, for single geometries
-    if ((long long)n * ngeom * 4 >= ONE_FEW)
+    if ((long long)n * ngeom * 4 >= 64ll * nsm)
         k_one_sp<LA, LB, 4><<<dim3((unsigned)((n * 4LL + 127) / 128), (unsigned)ngeom), 128>>>(a, pairs, n);
     else
         k_one_sp<LA, LB, 32><<<dim3((unsigned)((n * 32LL + 127) / 128), (unsigned)ngeom), 128>>>(a, pairs, n);
@@ -620,9 +619,12 @@ int one_electron_impl(const UnomolBasisDesc* b, const double* charges, int ngeom
         ck(cudaMemcpy(M, d_S.p, (size_t)9 * no2 * sizeof(double), cudaMemcpyDeviceToHost));
     } else if (e == cudaSuccess) {
         ck(boys_table());
-        launch_sp<1, 1>(a, pair_at[2], (int)pairs[2].size(), ngeom);
-        launch_sp<1, 0>(a, pair_at[1], (int)pairs[1].size(), ngeom);
-        launch_sp<0, 0>(a, pair_at[0], (int)pairs[0].size(), ngeom);
+        int dev = 0, nsm = 1;
+        ck(cudaGetDevice(&dev));
+        ck(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+        launch_sp<1, 1>(a, pair_at[2], (int)pairs[2].size(), ngeom, nsm);
+        launch_sp<1, 0>(a, pair_at[1], (int)pairs[1].size(), ngeom, nsm);
+        launch_sp<0, 0>(a, pair_at[0], (int)pairs[0].size(), ngeom, nsm);
         if (!items.empty()) {
             if (lmax == 2) k_one_electron<2><<<grid, 128>>>(a);
             else k_one_electron<4><<<grid, 128>>>(a);
