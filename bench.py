@@ -600,7 +600,7 @@ def run_ours(args):
                             "flush between calls (the value's device-timed builds each follow a 256 MiB flush)"},
             "roofline": {"bound": "fp64+fp32 pipes", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                          "frac": achieved / peak, "traffic": profile_traffic(args.form),
-                         "kernel": "fock_jk_kernel (all class instances and both precisions of a build)",
+                         "kernel": "fock_jk_kernel, fock_jk_group, fock_jk_df64 and fock_jk_*_part (all class instances of a build)",
                          "flops_fp64": fl64 / args.steps, "flops_fp32": fl32 / args.steps, "kernel_ms": 1e3 * eri_s / args.steps,
                          "peak_fp64": peak64, "peak_fp32": peak32,
                          "peak_note": "peak = (flops64 + flops32) / max(flops64 / peak64, flops32 / peak32): both pipes busy at once",

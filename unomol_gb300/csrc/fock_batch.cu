@@ -1,9 +1,10 @@
-// Batched Fock build over many molecules (the batching form): merged work lists, one persistent kernel
-// per quartet class pulling tiles from an atomic counter, the whole build captured as a CUDA graph,
-// and an autotuner choosing the CTA size (quartets per tile) and the CTAs per SM of every class.
-// RHF, shells up to d (the batch workload is s/p); FP64, or the precision form (per-build FP64 / FP32 /
-// skipped parts with each molecule's own density bound), whose two parts of a templated class run as
-// one grid launch with alternating CTAs.
+// Batched Fock build over many molecules (the batching form): merged work lists, the whole build captured
+// as a CUDA graph, and an autotuner choosing the CTA size (quartets per tile) and the CTAs per SM of every
+// class's persistent kernel, which pulls tiles from an atomic counter.  RHF, shells up to d (the batch
+// workload is s/p).  FP64: per class the quartets from SPLIT_CUT on with a few lanes each, the others in
+// pairs of floats (persistent).  The precision form (per-build FP64 / FP32 / skipped parts with each
+// molecule's own density bound): the FP64 part, its quartets in pairs of floats and the FP32 part
+// (persistent) as kernels of their own.
 #include <algorithm>
 #include <climits>
 #include <cstring>
@@ -26,7 +27,7 @@ template <int BC, int KC>
 cudaError_t persistent_one(const FockArgs& A, const NormTable& nt, const float* rys, int grid, int block, cudaStream_t s) {
     constexpr int LA = pc_la(BC), LB = pc_lb(BC), LC = pc_la(KC), LD = pc_lb(KC);
     if constexpr (QClass<LA, LB, LC, LD>::NF <= 81)
-        fock_jk_persistent<LA, LB, LC, LD, false, float><<<grid, block, 0, s>>>(A, nt, rys);
+        fock_jk_persistent<LA, LB, LC, LD><<<grid, block, 0, s>>>(A, nt, rys);
     else  // large classes: one item per thread over the whole launch
         fock_jk_generic<false, float, PrimPair32><<<(unsigned)((A.nwork + 63) / 64), 64, 0, s>>>(A, nt, rys, A.prims32, LA, LB, LC, LD);
     return cudaGetLastError();

@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(128, LA + LB + LC + LD <= 1 ? 8 : 1) fock_jk_d
     df_item<LA, LB, LC, LD, UHF>(A, nt, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-// The same for batches of molecules: a fixed grid pulling tiles (fock_jk_persistent).
+// The same for batches of molecules: a fixed grid pulling tiles (as fock_jk_persistent).
 template <int LA, int LB, int LC, int LD, bool UHF>
 __global__ void __launch_bounds__(256, LA + LB + LC + LD <= 1 ? 4 : 1) fock_jk_df64_persistent(const FockArgs A, const NormTable nt) {
     __shared__ long long tile;

@@ -10,7 +10,7 @@ static cudaError_t launch_one(const FockArgs& A, const NormTable& nt, const floa
     if (A.nwork <= 0) return cudaSuccess;
     if constexpr (QClass<LA, LB, LC, LD>::NF <= 81) {
         const long long blocks = (A.nwork + FOCK_THREADS - 1) / FOCK_THREADS;
-        fock_jk_kernel<LA, LB, LC, LD, UHF, float><<<(unsigned)blocks, FOCK_THREADS, 0, s>>>(A, nt, rys);
+        fock_jk_kernel<LA, LB, LC, LD, UHF><<<(unsigned)blocks, FOCK_THREADS, 0, s>>>(A, nt, rys);
     } else {
         const long long blocks = (A.nwork + 63) / 64;
         fock_jk_generic<UHF, float, PrimPair32><<<(unsigned)blocks, 64, 0, s>>>(A, nt, rys, A.prims32, LA, LB, LC, LD);

@@ -803,34 +803,23 @@ __device__ __forceinline__ void count_demoted(const FockArgs& A) {
                   (unsigned long long)__popc(m));
 }
 
-// Integrals, density contraction and scatter of one shell quartet in the arithmetic type R.
-template <int LA, int LB, int LC, int LD, bool UHF, typename R>
-__device__ __forceinline__ void quartet_item(const FockArgs& A, const NormTable& nt, const R* __restrict__ rys,
-                                             const ShellPair& bra, const ShellPair& ket, bool same_pair) {
-    using Q = QClass<LA, LB, LC, LD>;
-    unsigned npass = 0;
-    R acc[Q::NF];
-    if constexpr (sizeof(R) == 8)
-        shell_quartet_eri<LA, LB, LC, LD, R, PrimPair>(bra, ket, A.prims, rys, R(A.prim_cut), A.prim_cut32, A.rys_compat != 0, acc,
-                                                       A.counters ? &npass : nullptr);
-    else
-        shell_quartet_eri<LA, LB, LC, LD, R, PrimPair32>(bra, ket, A.prims32, rys, A.prim_cut32, A.prim_cut32, false, acc,
-                                                         A.counters ? &npass : nullptr);
-    digest_jk<LA, LB, LC, LD, UHF, R>(A, bra, ket, same_pair, acc, nt);
-    if (A.counters) count_flush(A, npass);
-}
-
-template <int LA, int LB, int LC, int LD, bool UHF, typename R>
-__device__ __forceinline__ void fock_item(const FockArgs& A, const NormTable& nt, const R* __restrict__ rys, long long g) {
+// One shell quartet of a screened build's FP32 part: integrals, density contraction and scatter by one lane.
+template <int LA, int LB, int LC, int LD, bool UHF>
+__device__ __forceinline__ void fock_item_fp32(const FockArgs& A, const NormTable& nt, const float* __restrict__ rys, long long g) {
     int bi, ki;
-    if (!(A.mode == 0 ? decode_work_warp<false>(A, g, bi, ki) : decode_work_warp<true>(A, g, bi, ki))) return;
+    if (!decode_work_warp<true>(A, g, bi, ki)) return;
     const ShellPair bra = A.pairs[bi];
     const ShellPair ket = A.pairs[ki];
-    if (A.mode != 0 && quartet_bound(A, bra, ket) < A.skip_cut32) {
+    if (quartet_bound(A, bra, ket) < A.skip_cut32) {
         if (A.counters) count_screened(A);
         return;
     }
-    quartet_item<LA, LB, LC, LD, UHF, R>(A, nt, rys, bra, ket, bi == ki);
+    unsigned npass = 0;
+    float acc[QClass<LA, LB, LC, LD>::NF];
+    shell_quartet_eri<LA, LB, LC, LD, float, PrimPair32>(bra, ket, A.prims32, rys, A.prim_cut32, A.prim_cut32, false, acc,
+                                                         A.counters ? &npass : nullptr);
+    digest_jk<LA, LB, LC, LD, UHF, float>(A, bra, ket, bi == ki, acc, nt);
+    if (A.counters) count_flush(A, npass);
 }
 
 // One shell quartet on a group of NP lanes (mask gmask): lane `part` of the group sums the primitive
@@ -857,26 +846,27 @@ __device__ __forceinline__ void quartet_item_group(const FockArgs& A, const Norm
     if (A.counters) count_flush(A, npass);
 }
 
-template <int LA, int LB, int LC, int LD, bool UHF, typename R>
-__global__ void __launch_bounds__(128) fock_jk_kernel(const FockArgs A, const NormTable nt, const R* __restrict__ rys) {
-    fock_item<LA, LB, LC, LD, UHF, R>(A, nt, rys, (long long)blockIdx.x * blockDim.x + threadIdx.x);
+// The FP32 part of one class.
+template <int LA, int LB, int LC, int LD, bool UHF>
+__global__ void __launch_bounds__(128) fock_jk_kernel(const FockArgs A, const NormTable nt, const float* __restrict__ rys) {
+    fock_item_fp32<LA, LB, LC, LD, UHF>(A, nt, rys, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // Persistent form for batches of molecules: a fixed grid of CTAs (a few per SM) pulls tiles of
 // blockDim consecutive work items from an atomic counter until the launch's work is done, so that
 // molecules of uneven size balance across the GPU in one launch per class.  Tiles follow the work
 // order (block pairs of one molecule are contiguous), which keeps a tile's warps uniform.
-template <int LA, int LB, int LC, int LD, bool UHF, typename R>
-__global__ void __launch_bounds__(256) fock_jk_persistent(const FockArgs A, const NormTable nt, const R* __restrict__ rys) {
+template <int LA, int LB, int LC, int LD>
+__global__ void __launch_bounds__(256) fock_jk_persistent(const FockArgs A, const NormTable nt, const float* __restrict__ rys) {
     __shared__ long long tile;
-    const long long end = A.mode != 0 ? *A.dyn_total : A.nwork;  // screened parts: their compact numbering
+    const long long end = *A.dyn_total;  // the part's compact numbering
     for (;;) {
         if (threadIdx.x == 0) tile = (long long)atomicAdd(A.tile_counter, 1ull);
         __syncthreads();
         const long long g0 = tile * blockDim.x;
         __syncthreads();
         if (g0 >= end) return;
-        fock_item<LA, LB, LC, LD, UHF, R>(A, nt, rys, g0 + threadIdx.x);
+        fock_item_fp32<LA, LB, LC, LD, false>(A, nt, rys, g0 + threadIdx.x);
     }
 }
 
