@@ -6,9 +6,9 @@
 //
 // What bounds it: the FP64 kernels keep the FP64 pipe (2 lanes per clock and SM) 88 % busy; the same
 // primitive quartet of (ps|ss) is about 65 FP64 instructions (1040 SM clocks per warp) or about 350 FP32
-// ones (88 clocks at full issue).  Here issue is 50-60 % active, the L1 data pipe 50-60 % and the FP64 pipe
-// (the density contraction) 17-33 %, with the loads the leading stall.  One build, GB300: 32 waters 6-31G
-// 74.6 -> 21.2 ms, n-decane cation UHF 12.1 -> 2.8 ms (with the group kernels below).
+// ones (88 clocks at full issue).  Here issue is 47-67 % active, the L1 data pipe 35-72 % and the FP64 pipe
+// (the density contraction) 16-36 %, with the loads the leading stall.  One build, GB300: 32 waters 6-31G
+// 79.3 -> 21.9 ms, n-decane cation UHF 12.2 -> 3.2 ms (with the group kernels below).
 // Measured beside it: look-ahead for the next surviving primitive quartet (as the FP64 kernels) instead of
 // plain loops, kept for la+lb+lc+ld = 2 only ((ps|ps) 3.9 against 4.2 ms, (ps|ss) 7.6 against 6.9); 64
 // registers for (ss|ss) and (ps|ss) (25.3 -> 24.0 ms for the build).
